@@ -179,6 +179,7 @@ int build_tables(hb_ctx *ctx, uint32_t logn, uint32_t logv, DevTables &t) {
   }
   const W ninv = hb::host_powmod<F>((W)N, order - 1);
   t.n_inv = F::to_mont(ninv);
+  t.psi = psi;
   // keys: mul(x, scale) must give x * N^-1 in the Montgomery domain of the key words
   t.key_scale = F::to_mont(F::to_mont(ninv));
   if (sizeof(W) == 8) t.key_scale = ninv;
@@ -245,6 +246,7 @@ uint32_t ks_dim(const hb_params &p) {
 // half-CTA groups (words per thread: hb::dp_wide_words).
 int dp_tables(hb_ctx *ctx, const hb_params &p, int T) {
   if (p.ring_dim != 1024) return HB_OK;
+  if (const int rc = tc_tables(ctx, p)) return rc;
   const int ws = p.field_id == HB_FIELD_GOLDILOCKS ? 8 : 4;
   for (int cl = 0; cl < 2; ++cl) {
     // hb::dp_group_threads, hb::dp_groups: the groups' own transforms and the half-CTA groups'
@@ -551,6 +553,13 @@ int launch_boot(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> &jobs, bool pla
   const GateJob *djobs = (const GateJob *)ctx->jobs.ptr;
   const unsigned grid = plain ? 1u : std::min<unsigned>(batches, (unsigned)ctx->sms);
   const unsigned block = G * T;
+  if constexpr (T == 128 && G == 4 && !TERN) {
+    if (!plain && !trace && tc_applies(keys->p, T, G)) {
+      rc = launch_tc(ctx, keys, djobs, (int)jobs.size(), batches, nullptr, ctx->stream);
+      if (!rc) ctx->launches += 1;
+      return rc;
+    }
+  }
   if (!plain) {
     prm.jobs = djobs;
     prm.njobs = (int)jobs.size();
@@ -647,6 +656,13 @@ int launch_table(hb_ctx *ctx, hb_keys *keys, const GateJob *djobs, int njobs, ui
   DevTables *tb;
   int rc = tables(ctx, F::FIELD_ID, LOGN, &tb, hb::GroupNtt<F, LOGN, T>::LOGV);
   if (rc) return rc;
+  if constexpr (T == 128 && G == 4 && !TERN) {
+    if (tc_applies(keys->p, T, G)) {
+      rc = launch_tc(ctx, keys, djobs, njobs, batches, nullptr, stream);
+      if (!rc) ctx->launches += 1;
+      return rc;
+    }
+  }
   hb::BootParams<W> prm{};
   boot_params(prm, ctx, keys, tb);
   prm.jobs = djobs;
@@ -1357,6 +1373,8 @@ int noalloc_gates_per_cta(const hb_keys *keys) {
 template <class F, int LOGN, int T, int G, bool TERN, bool KSC>
 int launch_noalloc(hb_ctx *ctx, hb_keys *keys, const DevTables *tb, const GateJob *djobs, int njobs,
                    uint32_t batches, int *dstatus) {
+  if constexpr (T == 128 && G == 4 && !TERN)
+    if (tc_applies(keys->p, T, G)) return launch_tc(ctx, keys, djobs, njobs, batches, dstatus, ctx->stream);
   using W = typename F::W;
   constexpr int N = 1 << LOGN;
   hb::BootParams<W> prm{};
@@ -1755,8 +1773,13 @@ int launch_gates_per_cta(const hb_ctx *ctx, const hb_keys *keys, uint64_t gates)
   std::vector<int> cand = variants(keys->p, keys->threads_per_gate);
   cand.push_back(1);
   std::sort(cand.begin(), cand.end());
-  for (int g : cand)
+  for (int g : cand) {
+    // The tensor-core form fills the smaller batched variants' place: a launch lasts one CTA's four gates
+    // whether they are there or not (GOLDILOCKS 46 ms), less than three gates in the other form (56 ms) and
+    // more than one in the latency form (18 ms).
+    if (g > 1 && g != tuned && tc_applies(keys->p, keys->threads_per_gate, tuned)) continue;
     if (g <= tuned && (gates + g - 1) / g <= sms) return g;
+  }
   return tuned;
 }
 

@@ -21,6 +21,7 @@ struct DevTables {
   void *itw = nullptr;  // psi^-brv(k), the same way
   unsigned long long n_inv = 0;      // multiplier giving x * N^-1
   unsigned long long key_scale = 0;  // multiplier applied to key words at upload
+  unsigned long long psi = 0;        // the primitive 2N-th root of the tables
 };
 
 struct Scratch {
@@ -40,6 +41,7 @@ struct hb_ctx {
   std::vector<std::pair<void *, size_t>> sizes;
   std::string err;
   hbrt::DevTables tables[3][13][6];  // [field][log2 N][log2 words per thread]
+  void *tc_tables = nullptr;                    // byte matrices of bootstrap_tc_kernel
   hbrt::Scratch jobs, io, mux_tmp;
   std::atomic<unsigned long long> launches{0};  // bootstrap kernel launches issued by this context
   long long wait_limit = 0;                     // SM clock cycles per bounded wait; 0 = default
@@ -76,6 +78,13 @@ uint32_t ks_dim(const hb_params &p);
 // One persistent bootstrapping launch over a device job table (full grid, the keys' variant).
 int launch_set(hb_ctx *ctx, hb_keys *keys, int gates_per_cta, const hb::GateJob *djobs, int njobs,
                uint32_t batches, cudaStream_t stream);
+// The tensor-core form of the persistent kernel (hb_boot_tc.cu): its tables, built with the keys;
+// whether it covers a parameter set under a (T, G) variant; one launch over a device job table in place
+// (status: another status word than the context's, or null).
+int tc_tables(hb_ctx *ctx, const hb_params &p);
+bool tc_applies(const hb_params &p, int T, int G);
+int launch_tc(hb_ctx *ctx, const hb_keys *keys, const hb::GateJob *djobs, int njobs, uint32_t batches, int *status,
+              cudaStream_t stream);
 int launch_gates_per_cta(const hb_ctx *ctx, const hb_keys *keys, uint64_t gates);
 // The job record of `count` single-bootstrap gates (NAND..MAJORITY) of parameter set p.
 int gate_job(const hb_params &p, int gate, const void *c0, const void *c1, const void *c2, void *out,
