@@ -709,18 +709,20 @@ __global__ void lwe_not_kernel(const typename F::W *in, typename F::W *out, size
 
 size_t word_size(const hb_params &p) { return p.field_id == HB_FIELD_GOLDILOCKS ? 8 : 4; }
 
-int default_threads_per_gate(int field_id) {
+int default_threads_per_gate(const hb_params &p) {
   const char *env = getenv("HB_THREADS_PER_GATE");
   if (env && (atoi(env) == 64 || atoi(env) == 128)) return atoi(env);
-  return field_id == HB_FIELD_GOLDILOCKS ? 128 : 64;  // measured best tiles on B200
+  // measured best tiles on B200; a ternary key's second set of sums makes 16 words a thread too many (700
+  // CUSTOM_TERNARY gates 29.1 ms at 64 threads, 24.6 at 128)
+  return p.field_id == HB_FIELD_GOLDILOCKS || p.lwe_ternary ? 128 : 64;
 }
 
 int default_gates_per_cta(int field_id) {
   const char *env = getenv("HB_GATES_PER_CTA");
   if (env && atoi(env) > 0) return atoi(env);
-  // measured best on B200 before autotuning: Goldilocks (T = 128) 4, BabyBear (T = 64, paired
-  // digit transforms) 8, DefaultFieldU32 (T = 64) 6
-  return field_id == HB_FIELD_GOLDILOCKS ? 4 : field_id == HB_FIELD_BABYBEAR ? 8 : 6;
+  // measured best on B200 before autotuning: Goldilocks (T = 128) 4, the 32-bit fields (T = 64) 8; 4 is all
+  // a ternary key's kernels hold
+  return field_id == HB_FIELD_GOLDILOCKS ? 4 : 8;
 }
 
 }  // namespace
@@ -824,7 +826,7 @@ int hb_keys_upload(hb_ctx *ctx, const hb_params *p, const void *bsk, const void 
     delete k;
     return rc;
   }
-  k->threads_per_gate = default_threads_per_gate(p->field_id);
+  k->threads_per_gate = default_threads_per_gate(*p);
   cudaError_t e = cudaMemcpyAsync(staging, bsk, nb * ws, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess)
     rc = prepare_field(ctx, p->field_id, logn, k->threads_per_gate, staging, k->bsk, nb / p->ring_dim);
@@ -1273,7 +1275,7 @@ extern "C" int hb_keys_generate(hb_ctx *ctx, const hb_params *p, uint64_t seed, 
   const size_t nkd = ksk_device_words(*p), ws = word_size(*p);
   hb_keys *k = new hb_keys();
   k->p = *p;
-  k->threads_per_gate = default_threads_per_gate(p->field_id);
+  k->threads_per_gate = default_threads_per_gate(*p);
   rc = dev_alloc(ctx, nb * ws, &k->bsk);
   if (!rc) rc = dev_alloc(ctx, nkd * ws, &k->ksk);
   if (!rc) {

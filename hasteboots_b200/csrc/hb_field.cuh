@@ -190,6 +190,8 @@ struct Goldilocks {
   // psi^e with e a multiple of N/32 is the power of two 2^(96 e / N) (GroupNtt::fwd_stage uses
   // ct_pow2 for those stages).
   static constexpr uint64_t SMALL_FIRST_GEN = 8;
+  static constexpr bool LAZY = false;
+  HB_HD static W tame(W x) { return x; }
   // The eighth roots of unity 2^24k make radix-8 passes cheaper than three radix-2 stages.
   static constexpr bool RADIX8 = true;
 };
@@ -277,8 +279,44 @@ struct Mont32 {
     x = add(u, v);
     y = shoup(sub(u, v), w.w, w.q);
   }
+  // LAZY (32 P < 2^32, DefaultFieldU32): the transforms skip the reductions of their sums and differences,
+  // since a Shoup product takes any 32-bit word and gives one below 2P. A forward butterfly then adds at
+  // most 2P to its larger input -- from canonical words, 23 P after the 11 stages of N = 2048 -- and an
+  // inverse one at most doubles it, so inverse passes of up to four stages start below 2P. 5 instructions a
+  // butterfly for about 10 (7104 gates on B200: DEFAULT_TERNARY 407.6 -> 340.9 ms, CUSTOM_TERNARY 105.9 ->
+  // 92.1; the multiply pipe, 74 % busy, bounds them now).
+  static constexpr bool LAZY = 32ull * PP < (1ull << 32);
+  static constexpr uint32_t FORWARD_BOUND = LAZY ? 24 : 1;  // forward transforms' outputs are below this times P
+  HB_HD static W shoup_lazy(W a, Tw w) {
+#ifdef __CUDA_ARCH__
+    const W h = __umulhi(a, w.q);
+#else
+    const W h = (W)(((uint64_t)a * w.q) >> 32);
+#endif
+    return a * w.w - h * P;
+  }
+  HB_HD static void ct_lazy(W &x, W &y, Tw w) {
+    const W t = shoup_lazy(y, w), u = x;
+    x = u + t;
+    y = u - t + 2 * P;
+  }
+  // y below bound P
+  HB_HD static void gs_lazy(W &x, W &y, Tw w, uint32_t bound) {
+    const W u = x, v = y;
+    x = u + v;
+    y = shoup_lazy(u - v + bound * P, w);
+  }
+  // Any 32-bit word to one below 2P of the same residue.
+  HB_HD static W tame(W x) {
+    if constexpr (LAZY) {
+      static_assert(!LAZY || ((1ull << BB) + (1ull << (32 - BB)) * ((1ull << BB) - PP) < 2ull * PP), "tame's bound");
+      return x - (x >> BB) * P;
+    } else {
+      return x;
+    }
+  }
   HB_HD static W mac(W acc, W x, W k) { return add(acc, mont(x, k)); }
-  // Sums of products x k (x, k < P) in the multiply-accumulate of the external product.
+  // Sums of products x k (x below FORWARD_BOUND P, k < P) in the multiply-accumulate of the external product.
   //  * WIDE (P < 2^28, DefaultFieldU32): t is a 64-bit sum of unreduced products, one 32x32 -> 64
   //    multiply-add each (10.8 % off a DEFAULT_TERNARY launch). fold() keeps t's residue and brings
   //    it below 2^32 (C + 1), C = 2^32 mod P, with one multiply-add, t_hi C + t_lo; FOLD products
@@ -291,7 +329,7 @@ struct Mont32 {
   static constexpr uint32_t C32 = (uint32_t)((1ull << 32) % PP);
   static constexpr bool WIDE = PP < (1u << 28);
   static constexpr int FOLD =
-      WIDE ? (int)((~0ull - (1ull << 32) * (C32 + 1ull)) / ((unsigned long long)PP * PP)) : (1 << 30);
+      WIDE ? (int)((~0ull - (1ull << 32) * (C32 + 1ull)) / ((unsigned long long)FORWARD_BOUND * PP * PP)) : (1 << 30);
   struct Acc {
     typename std::conditional<WIDE, uint64_t, uint32_t>::type t;
   };

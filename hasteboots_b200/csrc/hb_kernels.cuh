@@ -258,8 +258,12 @@ __global__ void __launch_bounds__(GPB * T) ntt_batch_kernel(const typename F::W 
     if (mode != 2) NT::forward(x, xbuf, ping, s_tw, t, sync);
     if (mode == 1) {
 #pragma unroll
-      for (int v = 0; v < V; ++v) dst[NT::slot_pos(t, v)] = F::canon(x[v]);
+      for (int v = 0; v < V; ++v) dst[NT::slot_pos(t, v)] = F::canon(F::tame(x[v]));
       continue;
+    }
+    if (mode == 0) {
+#pragma unroll
+      for (int v = 0; v < V; ++v) x[v] = F::tame(x[v]);
     }
     NT::inverse(x, xbuf, ping, s_itw, t, sync);
 #pragma unroll
@@ -503,7 +507,8 @@ constexpr bool kBootPingPong = HB_BOOT_PINGPONG != 0;
 // (16384 gates per launch), it pays for BabyBear where the launch leaves 128 registers per thread
 // (T G = 512 threads: T = 64, G = 8: 439.4 -> 427.7 ms; T = 128, G = 4: 501.7 -> 487.0 ms) and
 // costs elsewhere (BabyBear T = 64, G = 6: 447.9 -> 460.1 ms; DefaultFieldU32, whose 64-bit sums
-// already hold 32 more registers: up to 23 % slower), so only those variants use it.
+// already hold 32 more registers, no variant: DEFAULT_TERNARY T = 64, G = 6 340.2 -> 352.6 ms per 7104
+// gates, CUSTOM_TERNARY 90.8 -> 101.2 ms), so only those variants use it.
 template <class F, int T, int G>
 __host__ __device__ constexpr bool boot_dual() {
   if constexpr (sizeof(typename F::W) == 4) {
@@ -728,7 +733,8 @@ __global__ void __launch_bounds__(G * T, 1) bootstrap_kernel(const BootParams<ty
       auto mac_digit = [&](W(&x)[V]) -> bool {
         const W *k = pipe.acquire();
         if (active) {
-          if (fold_due<F>(nprod)) {
+          if (F::FOLD < (1 << 20) && nprod >= (uint32_t)F::FOLD) {
+            nprod = 0;
 #pragma unroll
             for (int v = 0; v < V; ++v) {
               F::acc_fold(acc_x[v]);
@@ -769,6 +775,14 @@ __global__ void __launch_bounds__(G * T, 1) bootstrap_kernel(const BootParams<ty
         const W *k0 = pipe.acquire();
         const W *k1 = pipe.acquire_next();
         if (active) {
+          if (F::FOLD < (1 << 20) && nprod + 2 > (uint32_t)F::FOLD) {
+            nprod = 0;
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+              F::acc_fold(acc_x[v]);
+              F::acc_fold(acc_y[v]);
+            }
+          }
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             F::acc_mac2(acc_x[v], x[v], k0[v * T + t], y[v], k1[v * T + t]);
@@ -801,7 +815,7 @@ __global__ void __launch_bounds__(G * T, 1) bootstrap_kernel(const BootParams<ty
             trace_digit(y, j + 1);
             NT::forward_small2(x, y, xbuf, ping, s_tw, t, sync);
           }
-          if constexpr (!TERN && !F::WIDE) {
+          if constexpr (!TERN) {
             if (!mac_pair(x, y)) goto aborted;
           } else {
             if (!mac_digit(x) || !mac_digit(y)) goto aborted;

@@ -15,6 +15,7 @@
 #pragma once
 
 #include "hb_field.cuh"
+#include "hb_sync.cuh"
 
 namespace hb {
 
@@ -191,6 +192,19 @@ struct GroupNtt {
     for (int k = 1; k < 8; ++k) x[k] = F::mul(x[k], th[(k - 1) << S0]);
   }
 
+  // A table entry in shared memory. The lazy butterflies are short, and the compiler would load all of a
+  // stage's twiddles ahead of them; loads that keep their order take no registers ahead of time (CUSTOM_TERNARY
+  // T = 64, G = 8 spilled 144 bytes a thread: 109.4 -> 92.1 ms per 7104 gates, DEFAULT_TERNARY 396 -> 341 ms).
+  __device__ __forceinline__ static TwT twiddle(const TwT *p) {
+    if constexpr (F::LAZY) {
+      uint32_t w, q;
+      asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w), "=r"(q) : "r"(smem_u32(p)));
+      return TwT{w, q};
+    } else {
+      return *p;
+    }
+  }
+
   // One forward (CT) stage on butterfly bit BB in a pass of layout LO. SMALL: inputs are words
   // below 2^15 (gadget digits) and this is the first stage, whose twiddle is 2^48.
   template <int LO, int BB, bool SMALL>
@@ -209,17 +223,30 @@ struct GroupNtt {
       const int base = (1 << S) + (t >> LO);
 #pragma unroll
       for (int k = 0; k < K; ++k) {
-        const TwT w = reinterpret_cast<const TwT *>(tw)[base + k * HIGHS];
+        const TwT w = twiddle(reinterpret_cast<const TwT *>(tw) + base + k * HIGHS);
 #pragma unroll
         for (int l = 0; l < (1 << RB); ++l) {
           const int v = (k << (RB + 1)) | l;
-          F::ct(x[v], x[v | (1 << RB)], w);
+          if constexpr (F::LAZY)
+            F::ct_lazy(x[v], x[v | (1 << RB)], w);
+          else
+            F::ct(x[v], x[v | (1 << RB)], w);
         }
       }
     }
   }
 
-  template <int LO, int BB>
+  // Lazy fields: register v is below this times P after the stages on register bits [rb0, rb) of an inverse
+  // pass that started below 2P (a product is below 2P, a sum below twice its inputs).
+  __host__ __device__ static constexpr uint32_t inv_bound(int v, int rb0, int rb) {
+    uint32_t b = 2;
+    while (rb > rb0 && !((v >> (rb - 1)) & 1)) {
+      b *= 2;
+      --rb;
+    }
+    return b;
+  }
+  template <int LO, int BB, int B0>
   __device__ __forceinline__ static void inv_stage(W (&x)[V], const W *__restrict__ itw, int t) {
     constexpr int RB = BB - LO;
     constexpr int H = N >> (BB + 1);
@@ -228,11 +255,14 @@ struct GroupNtt {
     const int base = H + (t >> LO);
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      const TwT w = reinterpret_cast<const TwT *>(itw)[base + k * HIGHS];
+      const TwT w = twiddle(reinterpret_cast<const TwT *>(itw) + base + k * HIGHS);
 #pragma unroll
       for (int l = 0; l < (1 << RB); ++l) {
         const int v = (k << (RB + 1)) | l;
-        F::gs(x[v], x[v | (1 << RB)], w);
+        if constexpr (F::LAZY)
+          F::gs_lazy(x[v], x[v | (1 << RB)], w, inv_bound(v, B0 - LO, RB));
+        else
+          F::gs(x[v], x[v | (1 << RB)], w);
       }
     }
   }
@@ -271,8 +301,15 @@ struct GroupNtt {
   __device__ __forceinline__ static void inv_stages(W (&x)[V], const W *itw, int t) {
     constexpr int LO = B0 < LOGN - LOGV ? B0 : LOGN - LOGV;
     constexpr int END = B0 + LOGV < LOGN ? B0 + LOGV : LOGN;
-    inv_stage<LO, BB>(x, itw, t);
-    if constexpr (BB + 1 < END) inv_stages<B0, BB + 1>(x, itw, t);
+    inv_stage<LO, BB, B0>(x, itw, t);
+    if constexpr (BB + 1 < END) {
+      inv_stages<B0, BB + 1>(x, itw, t);
+    } else if constexpr (F::LAZY) {
+      static_assert(END - B0 <= 4, "sums of more than four stages can exceed 32 P");
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        if (inv_bound(v, B0 - LO, END - LO) > 2) x[v] = F::tame(x[v]);
+    }
   }
   template <int B0>
   __device__ __forceinline__ static void inv_pass(W (&x)[V], W *buf, int &ping, const W *itw, int t,
@@ -336,7 +373,9 @@ struct GroupNtt {
                                                        int t, const GroupSync<T> &sync) {
     fwd_pass<LOGN, true>(x, buf, ping, tw, t, sync);
   }
-  // x: slots at slot_pos(t, v) -> N * (natural-order values) at natural_pos(t, v).
+  // x: slots at slot_pos(t, v), canonical (lazy fields: below 2P) -> N * (natural-order values) at
+  // natural_pos(t, v) (32-bit lazy fields: below 2P). Forward outputs of a lazy field are below
+  // F::FORWARD_BOUND P.
   __device__ __forceinline__ static void inverse(W (&x)[V], W *buf, int &ping, const W *itw, int t,
                                                  const GroupSync<T> &sync) {
     inv_pass<0>(x, buf, ping, itw, t, sync);
