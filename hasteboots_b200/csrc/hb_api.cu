@@ -522,21 +522,17 @@ int launch_dp(hb_ctx *ctx, hb::BootParams<typename F::W> prm, cudaStream_t strea
   return launch_dp_c<F, LOGN, T, 1, KSC, TERN>(ctx, prm, stream, nullptr);
 }
 
-template <class F, int LOGN, int T, int G, bool TERN, bool KSC>
+// One gate per launch: the plain form (one launch per job, one job per gate), or a traced gate in the latency
+// form.
+template <class F, int LOGN, int T, bool TERN, bool KSC>
 int launch_boot(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> &jobs, bool plain, void *trace) {
   using W = typename F::W;
-  constexpr int N = 1 << LOGN;
+  constexpr int N = 1 << LOGN, G = 1;
   DevTables *tb;
   int rc = tables(ctx, F::FIELD_ID, LOGN, &tb, hb::GroupNtt<F, LOGN, T>::LOGV);
   if (rc) return rc;
-  // Batched: jobs are laid end to end in batch space. Plain: every launch holds one job whose
-  // batches start at 0.
-  uint32_t batches = 0;
-  for (auto &j : jobs) {
-    j.first_batch = plain ? 0 : batches;
-    batches += (j.count + G - 1) / G;
-  }
-  if (batches == 0) return HB_OK;
+  if (jobs.empty()) return HB_OK;
+  for (auto &j : jobs) j.first_batch = 0;
   rc = scratch(ctx, ctx->jobs, sizeof(GateJob) * jobs.size());
   if (rc) return rc;
   cudaError_t e = cudaMemcpyAsync(ctx->jobs.ptr, jobs.data(), sizeof(GateJob) * jobs.size(),
@@ -544,40 +540,23 @@ int launch_boot(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> &jobs, bool pla
   if (e != cudaSuccess) return cuda_fail(ctx, e, "job table upload");
   hb::BootParams<W> prm{};
   boot_params(prm, ctx, keys, tb);
-  prm.trace = (W *)trace;
+  const GateJob *djobs = (const GateJob *)ctx->jobs.ptr;
+  prm.njobs = 1;
+  prm.total_batches = 1;
+  if (!plain) {
+    prm.trace = (W *)trace;
+    prm.jobs = djobs;
+    return launch_dp<F, LOGN, T, KSC, TERN>(ctx, prm, ctx->stream);
+  }
   constexpr int S = hb::boot_stages<W, N, G>();
   auto kern = hb::bootstrap_kernel<F, LOGN, T, G, S, TERN, KSC>;
   const size_t smem = hb::boot_smem_bytes<W, N, G, S>(prm.n);
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "bootstrap smem attribute");
-  const GateJob *djobs = (const GateJob *)ctx->jobs.ptr;
-  const unsigned grid = plain ? 1u : std::min<unsigned>(batches, (unsigned)ctx->sms);
-  const unsigned block = G * T;
-  if constexpr (T == 128 && G == 4 && !TERN) {
-    if (!plain && !trace && tc_applies(keys->p, T, G)) {
-      rc = launch_tc(ctx, keys, djobs, (int)jobs.size(), batches, nullptr, ctx->stream);
-      if (!rc) ctx->launches += 1;
-      return rc;
-    }
-  }
-  if (!plain) {
-    prm.jobs = djobs;
-    prm.njobs = (int)jobs.size();
-    prm.total_batches = batches;
-    if constexpr (G == 1) return launch_dp<F, LOGN, T, KSC, TERN>(ctx, prm, ctx->stream);
-    kern<<<grid, block, smem, ctx->stream>>>(prm);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "bootstrap launch");
-    ctx->launches += 1;
-    return HB_OK;
-  }
-  // plain form: one launch per job (each job is one gate)
   for (size_t i = 0; i < jobs.size(); ++i) {
     prm.jobs = djobs + i;
-    prm.njobs = 1;
-    prm.total_batches = 1;
     hb::BootParams<W> one = prm;
-    kern<<<1, block, smem, ctx->stream>>>(one);
+    kern<<<1, G * T, smem, ctx->stream>>>(one);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "bootstrap launch");
     ctx->launches += 1;
@@ -611,20 +590,24 @@ int launch_boot(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> &jobs, bool pla
 template <class F>
 constexpr int field_of() { return F::FIELD_ID; }
 
+int run_rounds(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> jobs);
+
 // trace: the accumulator trace of a one-gate launch (the latency form records it), or null.
 int run_jobs(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> &jobs, bool plain, void *trace = nullptr) {
   if (keys->p.ring_dim != 1024)
     return fail(ctx, HB_ERR_UNSUPPORTED, "bootstrapping is compiled for N = 1024");
   uint64_t gates = 0;
   for (auto &j : jobs) gates += j.count;
+  if (!plain && !trace) return run_rounds(ctx, keys, jobs);
   const int G = plain ? 1 : launch_gates_per_cta(ctx, keys, gates), T = keys->threads_per_gate,
             fld = keys->p.field_id;
   const bool tern = keys->p.lwe_ternary != 0, ksc = ks_dim(keys->p) < keys->p.ring_dim;
   if (trace && (plain || G != 1 || tern || gates != 1))
     return fail(ctx, HB_ERR_UNSUPPORTED, "accumulator traces are recorded for one gate under a binary LWE key");
+  for (auto &j : jobs) j.per_batch = 1;
 #define HB_CASE(FLD, TT, GG, TN, KC)                                             \
-  if (fld == field_of<FLD>() && T == TT && G == GG && tern == TN && ksc == KC) \
-    return launch_boot<FLD, 10, TT, GG, TN, KC>(ctx, keys, jobs, plain, trace);
+  if (GG == 1 && fld == field_of<FLD>() && T == TT && tern == TN && ksc == KC) \
+    return launch_boot<FLD, 10, TT, TN, KC>(ctx, keys, jobs, plain, trace);
   HB_BOOT_VARIANTS(HB_CASE)
 #undef HB_CASE
   return fail(ctx, HB_ERR_UNSUPPORTED, "no compiled kernel with %d threads per gate and %d gates per CTA", T, G);
@@ -692,6 +675,83 @@ int launch_table_any(hb_ctx *ctx, hb_keys *keys, int G, const GateJob *djobs, in
   HB_BOOT_VARIANTS(HB_CASE)
 #undef HB_CASE
   return fail(ctx, HB_ERR_UNSUPPORTED, "no compiled kernel with %d threads per gate and %d gates per CTA", T, G);
+}
+
+// Cuts the front of a job list, at most `batches` batches of `per` gates (batches do not span jobs), off into
+// `front`; what is left stays in `jobs`.
+void cut_front(const hb_params &p, std::vector<GateJob> &jobs, uint64_t batches, uint32_t per, std::vector<GateJob> &front) {
+  const size_t bytes = ((size_t)p.lwe_dim + 1) * (p.field_id == HB_FIELD_GOLDILOCKS ? 8 : 4);
+  std::vector<GateJob> left;
+  for (GateJob j : jobs) {
+    GateJob f = j;
+    f.count = (uint32_t)std::min<uint64_t>(j.count, batches * per);
+    f.per_batch = per;
+    batches -= (f.count + per - 1) / per;
+    if (f.count) front.push_back(f);
+    if (f.count == j.count) continue;
+    for (const void **in : {&j.in0, &j.in1, &j.in2})
+      if (*in) *in = (const char *)*in + f.count * bytes;
+    j.out = (char *)j.out + f.count * bytes;
+    j.count -= f.count;
+    left.push_back(j);
+  }
+  jobs = left;
+}
+
+uint64_t batch_sum(const std::vector<GateJob> &jobs, uint64_t per) {
+  uint64_t b = 0;
+  for (auto &j : jobs) b += (j.count + per - 1) / per;
+  return b;
+}
+
+// Gate calls of one key set: whole rounds of the tuned variant in one launch, and the gates after them, too few
+// for a round, in a second one of a shape of their own: spread evenly over all SMs in the smallest variant
+// that holds them, or in the latency form when that is one gate per SM. (In the last round of one launch
+// they held a few SMs for a full round while the others idled. B200, one launch -> this: 1300 BABYBEAR
+// gates 48.2 -> 29.3 ms, 2500 BABYBEAR 72.3 -> 53.8, 600 GOLDILOCKS 92.4 -> 56.4.)
+int run_rounds(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> jobs) {
+  const uint32_t tuned = (uint32_t)keys->gates_per_cta;
+  const uint64_t sms = (uint64_t)std::max(1, ctx->sms);
+  std::vector<GateJob> table;
+  cut_front(keys->p, jobs, batch_sum(jobs, tuned) / sms * sms, tuned, table);
+  uint64_t rest = 0;
+  for (auto &j : jobs) rest += j.count;
+  uint64_t even = (rest + sms - 1) / sms;  // gates per SM of the rest, in at most one batch per SM
+  while (rest && batch_sum(jobs, even) > sms) ++even;
+  // The tensor-core form lasts its four gates whether they are there or not; and one gate short of a full CTA
+  // does not pay in the other form (its idle group polls for keys: 900 BABYBEAR gates seven to a CTA 24.7 ms,
+  // eight 24.2).
+  if (even > 1 && (even + 1 >= tuned || tc_applies(keys->p, keys->threads_per_gate, (int)tuned)))
+    cut_front(keys->p, jobs, ~0ull / tuned, tuned, table);
+  const size_t first = table.size();
+  int rest_variant = even <= 1 ? 1 : (int)tuned;
+  if (jobs.size()) {
+    if (even > 1)
+      for (int g : variants(keys->p, keys->threads_per_gate))
+        if ((uint64_t)g >= even && g < rest_variant) rest_variant = g;
+    if (even + 1 >= (uint64_t)rest_variant) even = rest_variant;
+    cut_front(keys->p, jobs, ~0ull / tuned, (uint32_t)even, table);
+  }
+  if (table.empty()) return HB_OK;
+  uint32_t batches[2] = {0, 0};
+  for (size_t i = 0; i < table.size(); ++i) {
+    GateJob &j = table[i];
+    uint32_t &b = batches[i < first ? 0 : 1];
+    j.first_batch = b;
+    b += (j.count + j.per_batch - 1) / j.per_batch;
+  }
+  int rc = scratch(ctx, ctx->jobs, sizeof(GateJob) * table.size());
+  if (rc) return rc;
+  const cudaError_t e = cudaMemcpyAsync(ctx->jobs.ptr, table.data(), sizeof(GateJob) * table.size(),
+                                        cudaMemcpyHostToDevice, ctx->stream);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "job table upload");
+  const GateJob *djobs = (const GateJob *)ctx->jobs.ptr;
+  if (batches[0])
+    rc = launch_table_any(ctx, keys, tuned, djobs, (int)first, batches[0], (unsigned)ctx->sms, ctx->stream);
+  if (!rc && batches[1])
+    rc = launch_table_any(ctx, keys, rest_variant, djobs + first, (int)(table.size() - first), batches[1],
+                          (unsigned)ctx->sms, ctx->stream);
+  return rc;
 }
 
 bool single_bootstrap_gate(int gate) { return gate >= HB_GATE_NAND && gate <= HB_GATE_MAJORITY; }
@@ -1453,6 +1513,7 @@ extern "C" int hb_gate_mux_device_noalloc(hb_ctx *ctx, hb_keys *keys, const void
   jobs[0].first_batch = 0;
   jobs[1].first_batch = per_job;
   jobs[2].first_batch = 0;
+  for (GateJob &j : jobs) j.per_batch = (uint32_t)G;
 
   // The array keeps the previous call's contents: the status word must start at zero.
   e = cudaMemsetAsync(dstatus, 0, sizeof(int), ctx->stream);
@@ -1582,6 +1643,7 @@ extern "C" int hb_autotune(hb_ctx *ctx, hb_keys *keys, uint32_t sample_gates, in
     std::vector<GateJob> jobs{make_job(modulus_of(keys->p.field_id), HB_GATE_NAND, 1024, buf, buf,
                                        nullptr, (char *)buf + bytes, sample_gates)};
     jobs[0].first_batch = 0;
+    jobs[0].per_batch = (uint32_t)G;
     const uint32_t batches = batches_of(jobs, G);
     cudaMemcpyAsync(tab, jobs.data(), sizeof(GateJob), cudaMemcpyHostToDevice, ctx->stream);
     float best_ms = 1e30f;
@@ -1692,6 +1754,7 @@ extern "C" int hb_batch_create(hb_ctx *ctx, const hb_job *jobs, size_t njobs, hb
     uint32_t bsum = 0;
     for (auto &t : tab) {
       t.first_batch = bsum;
+      t.per_batch = (uint32_t)G;
       bsum += (t.count + G - 1) / G;
     }
     grp.batches = bsum;

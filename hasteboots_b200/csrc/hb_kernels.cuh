@@ -71,6 +71,7 @@ struct GateJob {
   int32_t s0, s1, s2;
   uint32_t count;
   uint32_t first_batch;
+  uint32_t per_batch;  // gates per batch, at most the kernel's G (bootstrap_kernel; the other forms: fixed)
 };
 
 // Ring of S shared-memory stages fed by the TMA unit with consecutive 2N-word chunks of key
@@ -617,8 +618,8 @@ __global__ void __launch_bounds__(G * T, 1) bootstrap_kernel(const BootParams<ty
     int jx = 0;
     while (jx + 1 < p.njobs && p.jobs[jx + 1].first_batch <= batch) ++jx;
     const GateJob &job = p.jobs[jx];
-    const uint32_t gate = (batch - job.first_batch) * G + g;
-    const bool active = gate < job.count;
+    const uint32_t gate = (batch - job.first_batch) * job.per_batch + g;
+    const bool active = (uint32_t)g < job.per_batch && gate < job.count;
     const size_t lwe_words = (size_t)n + 1;
 
     // ---- input combine + modulus switch (Evaluator::nand etc., evaluate.rs:113-119) ----

@@ -181,6 +181,7 @@ int launch_wave(hb_server *s, std::vector<Request *> reqs, int slot) {
     uint32_t batches = 0;
     for (auto &j : tabs[k]) {
       j.first_batch = batches;
+      j.per_batch = (uint32_t)G;
       batches += (j.count + G - 1) / G;
     }
     cudaStream_t st = s->set_streams[slot * kMaxSets + k];

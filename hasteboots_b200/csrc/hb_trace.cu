@@ -86,6 +86,7 @@ extern "C" int hb_bootstrap_trace_device(hb_ctx *ctx, hb_keys *keys, const void 
   job.s0 = 1;
   job.count = (uint32_t)count;
   job.first_batch = 0;
+  job.per_batch = kTraceGates;
   int rc = scratch(ctx, ctx->jobs, sizeof(GateJob));
   if (rc) return rc;
   e = cudaMemcpyAsync(ctx->jobs.ptr, &job, sizeof(GateJob), cudaMemcpyHostToDevice, ctx->stream);
