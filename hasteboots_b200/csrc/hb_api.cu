@@ -246,7 +246,7 @@ uint32_t ks_dim(const hb_params &p) {
 // half-CTA groups (words per thread: hb::dp_wide_words).
 int dp_tables(hb_ctx *ctx, const hb_params &p, int T) {
   if (p.ring_dim != 1024) return HB_OK;
-  if (const int rc = tc_tables(ctx, p)) return rc;
+  tc_tables(ctx, p.field_id, p.ring_dim);
   const int ws = p.field_id == HB_FIELD_GOLDILOCKS ? 8 : 4;
   for (int cl = 0; cl < 2; ++cl) {
     // hb::dp_group_threads, hb::dp_groups: the groups' own transforms and the half-CTA groups'
@@ -362,11 +362,13 @@ int launch_ext(hb_ctx *ctx, const void *rgsw, uint32_t bits, uint32_t len, const
   const size_t smem = sizeof(W) * (2 * hb::tw_words<W>() * N + kStages * 2 * N + G * 2 * N) + sizeof(uint64_t) * kStages +
                       2 * sizeof(uint32_t) * kStages + 16;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const size_t batches = (count + G - 1) / G;
+  // RLWEs per CTA: fewer than G while SMs would be idle (148 BABYBEAR RLWEs, N = 1024: 24.7 us with four, 14.6
+  // with one)
+  const size_t per = std::min<size_t>(G, (count + ctx->sms - 1) / ctx->sms), batches = (count + per - 1) / per;
   const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>(batches, (size_t)ctx->sms));
   kern<<<grid, G * T, smem, ctx->stream>>>((const W *)in, (W *)out, count, (const W *)rgsw, len, bits,
                                             (const W *)tb->tw, (const W *)tb->itw, ctx->d_status,
-                                            wait_budget(ctx));
+                                            wait_budget(ctx), (uint32_t)per);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? HB_OK : cuda_fail(ctx, e, "external product launch");
 }
@@ -640,7 +642,7 @@ int launch_table(hb_ctx *ctx, hb_keys *keys, const GateJob *djobs, int njobs, ui
   int rc = tables(ctx, F::FIELD_ID, LOGN, &tb, hb::GroupNtt<F, LOGN, T>::LOGV);
   if (rc) return rc;
   if constexpr (T == 128 && G == 4 && !TERN) {
-    if (tc_applies(keys->p, T, G)) {
+    if (tc_applies(ctx, keys->p, T, G)) {
       rc = launch_tc(ctx, keys, djobs, njobs, batches, nullptr, stream);
       if (!rc) ctx->launches += 1;
       return rc;
@@ -721,7 +723,7 @@ int run_rounds(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> jobs) {
   // The tensor-core form lasts its four gates whether they are there or not; and one gate short of a full CTA
   // does not pay in the other form (its idle group polls for keys: 900 BABYBEAR gates seven to a CTA 24.7 ms,
   // eight 24.2).
-  if (even > 1 && (even + 1 >= tuned || tc_applies(keys->p, keys->threads_per_gate, (int)tuned)))
+  if (even > 1 && (even + 1 >= tuned || tc_applies(ctx, keys->p, keys->threads_per_gate, (int)tuned)))
     cut_front(keys->p, jobs, ~0ull / tuned, tuned, table);
   const size_t first = table.size();
   int rest_variant = even <= 1 ? 1 : (int)tuned;
@@ -1139,6 +1141,7 @@ int hb_rgsw_upload(hb_ctx *ctx, int field_id, uint32_t log_n, uint32_t bits, uin
   }
   cudaMemcpyAsync(staging, rgsw, words * ws, cudaMemcpyHostToDevice, ctx->stream);
   rc = prepare_field(ctx, field_id, log_n, std_threads(log_n), staging, dst, words / N);
+  if (!rc) tc_tables(ctx, field_id, (uint32_t)N);
   cudaError_t e = cudaStreamSynchronize(ctx->stream);
   dev_free(ctx, staging);
   if (rc || e != cudaSuccess) {
@@ -1164,7 +1167,25 @@ int hb_external_product_device(hb_ctx *ctx, int field_id, uint32_t log_n, uint32
   if (count == 0) return HB_OK;
   cudaSetDevice(ctx->device);
   if (field_id == HB_FIELD_GOLDILOCKS) {
-    if (log_n == 10) return launch_ext<Goldilocks, 10, 128, 4>(ctx, d_rgsw, bits, len, rlwe_in, rlwe_out, count);
+    if (log_n == 10) {
+      // The tensor-core form (digits of a byte) lasts four RLWEs per SM whether they are there or not, so whole
+      // rounds of four go to it and a rest of more than two; a rest of one or two per SM is shorter in the
+      // butterfly form. l = 13, B = 2^5 on B200, butterfly / tensor form: 148 RLWEs 66 / 98 us, 296 93 / 99,
+      // 444 122 / 99, 592 153 / 100, 4096 994 / 677.
+      size_t rest = count;
+      if (bits <= 8 && ctx->tc_tables) {
+        const size_t sms = (size_t)ctx->sms;
+        rest = count % (4 * sms);
+        if (rest > 2 * sms) rest = 0;
+        if (count > rest) {
+          const int rc = launch_tc_ext(ctx, d_rgsw, bits, len, rlwe_in, rlwe_out, count - rest);
+          if (rc || rest == 0) return rc;
+        }
+      }
+      const size_t at = (count - rest) * 2 * 1024;
+      return launch_ext<Goldilocks, 10, 128, 4>(ctx, d_rgsw, bits, len, (const uint64_t *)rlwe_in + at,
+                                                (uint64_t *)rlwe_out + at, rest);
+    }
     if (log_n == 11) return launch_ext<Goldilocks, 11, 256, 2>(ctx, d_rgsw, bits, len, rlwe_in, rlwe_out, count);
   } else if (field_id == HB_FIELD_BABYBEAR) {
     if (log_n == 10) return launch_ext<BabyBear, 10, 128, 4>(ctx, d_rgsw, bits, len, rlwe_in, rlwe_out, count);
@@ -1436,7 +1457,7 @@ template <class F, int LOGN, int T, int G, bool TERN, bool KSC>
 int launch_noalloc(hb_ctx *ctx, hb_keys *keys, const DevTables *tb, const GateJob *djobs, int njobs,
                    uint32_t batches, int *dstatus) {
   if constexpr (T == 128 && G == 4 && !TERN)
-    if (tc_applies(keys->p, T, G)) return launch_tc(ctx, keys, djobs, njobs, batches, dstatus, ctx->stream);
+    if (tc_applies(ctx, keys->p, T, G)) return launch_tc(ctx, keys, djobs, njobs, batches, dstatus, ctx->stream);
   using W = typename F::W;
   constexpr int N = 1 << LOGN;
   hb::BootParams<W> prm{};
@@ -1842,7 +1863,7 @@ int launch_gates_per_cta(const hb_ctx *ctx, const hb_keys *keys, uint64_t gates)
     // The tensor-core form fills the smaller batched variants' place: a launch lasts one CTA's four gates
     // whether they are there or not (GOLDILOCKS 46 ms), less than three gates in the other form (56 ms) and
     // more than one in the latency form (18 ms).
-    if (g > 1 && g != tuned && tc_applies(keys->p, keys->threads_per_gate, tuned)) continue;
+    if (g > 1 && g != tuned && tc_applies(ctx, keys->p, keys->threads_per_gate, tuned)) continue;
     if (g <= tuned && (gates + g - 1) / g <= sms) return g;
   }
   return tuned;

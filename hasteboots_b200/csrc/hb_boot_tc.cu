@@ -56,39 +56,36 @@ std::vector<unsigned char> build_tc(uint64_t psi) {
   return t;
 }
 
-template <bool KSC>
-int launch(hb_ctx *ctx, const hb::BootParams<uint64_t> &prm, const unsigned char *tab, cudaStream_t stream) {
-  auto kern = hb::bootstrap_tc_kernel<KSC>;
+template <bool KSC, bool EXT = false>
+int launch(hb_ctx *ctx, const hb::BootParams<uint64_t> &prm, const unsigned char *tab, cudaStream_t stream,
+           const hb::TcExt &ext = {}) {
+  auto kern = hb::bootstrap_tc_kernel<KSC, EXT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Geo::SMEM);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "bootstrap smem attribute");
   const unsigned grid = std::max(1u, std::min<unsigned>(prm.total_batches, (unsigned)ctx->sms));
-  kern<<<grid, Geo::THREADS + Geo::AUX, Geo::SMEM, stream>>>(prm, tab);
+  kern<<<grid, Geo::THREADS + Geo::AUX, Geo::SMEM, stream>>>(prm, tab, ext);
   e = cudaGetLastError();
   return e == cudaSuccess ? HB_OK : cuda_fail(ctx, e, "bootstrap launch");
 }
 
 }  // namespace
 
-int tc_tables(hb_ctx *ctx, const hb_params &p) {
-  if (ctx->tc_tables || p.field_id != HB_FIELD_GOLDILOCKS || p.ring_dim != Geo::N) return HB_OK;
+void tc_tables(hb_ctx *ctx, int field_id, uint32_t ring_dim) {
+  if (ctx->tc_tables || field_id != HB_FIELD_GOLDILOCKS || ring_dim != Geo::N) return;
   DevTables *tb;
-  int rc = tables(ctx, p.field_id, Geo::LOGN, &tb, 3);
-  if (rc) return rc;
+  if (tables(ctx, field_id, Geo::LOGN, &tb, 3)) return;
   const std::vector<unsigned char> t = build_tc(tb->psi);
   void *d = nullptr;
-  rc = dev_alloc(ctx, t.size(), &d);
-  if (rc) return rc;
-  const cudaError_t e = cudaMemcpy(d, t.data(), t.size(), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) {
+  if (dev_alloc(ctx, t.size(), &d)) return;
+  if (cudaMemcpy(d, t.data(), t.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
     dev_free(ctx, d);
-    return cuda_fail(ctx, e, "tensor table upload");
+    return;
   }
   ctx->tc_tables = d;
-  return HB_OK;
 }
 
-bool tc_applies(const hb_params &p, int T, int G) {
-  return p.field_id == HB_FIELD_GOLDILOCKS && T == 128 && G == Geo::G && !p.lwe_ternary && p.ring_dim == Geo::N &&
+bool tc_applies(const hb_ctx *ctx, const hb_params &p, int T, int G) {
+  return ctx->tc_tables && p.field_id == HB_FIELD_GOLDILOCKS && T == 128 && G == Geo::G && !p.lwe_ternary && p.ring_dim == Geo::N &&
          p.br_bits <= 8 && p.ks_bits <= 8;
 }
 
@@ -96,7 +93,6 @@ int launch_tc(hb_ctx *ctx, const hb_keys *keys, const GateJob *djobs, int njobs,
               cudaStream_t stream) {
   const DevTables *tb = &ctx->tables[HB_FIELD_GOLDILOCKS][Geo::LOGN][3];  // built with the keys, as the tensor tables
   const unsigned char *tab = (const unsigned char *)ctx->tc_tables;
-  if (!tb->tw || !tab) return fail(ctx, HB_ERR_INVALID, "keys were not prepared on this context");
   hb::BootParams<uint64_t> prm{};
   boot_params(prm, ctx, keys, tb);
   prm.jobs = djobs;
@@ -104,6 +100,29 @@ int launch_tc(hb_ctx *ctx, const hb_keys *keys, const GateJob *djobs, int njobs,
   prm.total_batches = batches;
   if (status) prm.status = status;
   return ks_dim(keys->p) < keys->p.ring_dim ? launch<true>(ctx, prm, tab, stream) : launch<false>(ctx, prm, tab, stream);
+}
+
+int launch_tc_ext(hb_ctx *ctx, const void *rgsw, uint32_t bits, uint32_t len, const void *in, void *out, size_t count) {
+  const DevTables *tb = &ctx->tables[HB_FIELD_GOLDILOCKS][Geo::LOGN][3];
+  const unsigned char *tab = (const unsigned char *)ctx->tc_tables;
+  hb::BootParams<uint64_t> prm{};
+  prm.bsk = (const uint64_t *)rgsw;
+  prm.tw = (const uint64_t *)tb->tw;
+  prm.itw = (const uint64_t *)tb->itw;
+  prm.len = len;
+  prm.bits = bits;
+  prm.status = ctx->d_status;
+  prm.budget = wait_budget(ctx);
+  // at most 2^32 - 1 batches a launch
+  for (size_t at = 0; at < count;) {
+    const size_t part = std::min(count - at, (size_t)0xFFFFFF00u * Geo::G);
+    prm.total_batches = (uint32_t)((part + Geo::G - 1) / Geo::G);
+    const int rc = launch<false, true>(ctx, prm, tab, ctx->stream,
+                                       {(const uint64_t *)in + at * 2 * Geo::N, (uint64_t *)out + at * 2 * Geo::N, part});
+    if (rc) return rc;
+    at += part;
+  }
+  return HB_OK;
 }
 
 }  // namespace hbrt

@@ -209,9 +209,17 @@ __device__ __forceinline__ uint32_t tc_digits4(const uint64_t *x, uint32_t sh, u
 
 // Same bootstrap, jobs and keys (T = 128 layout) as bootstrap_kernel with G = 4 over Goldilocks and a binary
 // LWE key; gadget and key-switch bases up to 2^8. tab: the tensor tables (TcGeo::TAB_BYTES). KSC as there.
-template <bool KSC>
+//
+// EXT: external products instead (ext_product_kernel): ext's RLWEs, four to a batch, times the RGSW at p.bsk --
+// one step without a rotation or an accumulator, its E read from global memory.
+struct TcExt {
+  const uint64_t *in;
+  uint64_t *out;
+  unsigned long long count;
+};
+template <bool KSC, bool EXT = false>
 __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
-    bootstrap_tc_kernel(const BootParams<uint64_t> p, const unsigned char *__restrict__ tab) {
+    bootstrap_tc_kernel(const BootParams<uint64_t> p, const unsigned char *__restrict__ tab, const TcExt ext) {
   using F = Goldilocks;
   using W = uint64_t;
   using Geo = TcGeo;
@@ -257,7 +265,7 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
   W *acc_a = s_acc + g * 2 * N, *acc_b = acc_a + N;
   W *xbuf = reinterpret_cast<W *>(s_a2) + g * (N + Geo::XPAD);
   uint16_t *ms = s_ms + g * Geo::MS_STEPS;
-  const uint32_t n = p.n;
+  const uint32_t n = EXT ? 0 : p.n;  // EXT: step 0 alone
   const uint32_t ks_chunks = KSC ? p.ks_chunks : 1;
   // pairs of digits per part (a blind-rotation step has parts E.a and E.b, the key switch one per chunk)
   const uint32_t br_pairs = (p.len + 1) / 2, ks_pairs = (p.ks_len + 1) / 2;
@@ -304,8 +312,9 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
       uint32_t groups = 0;
       for (uint32_t b = 0; b < my_batches; ++b)
         for (uint32_t step = 0; step <= n; ++step) {
-          const uint32_t L = step == n ? p.ks_len : p.len, pairs = (L + 1) / 2;
-          const uint32_t units = step == n ? ks_units : br_units;
+          const bool ks = !EXT && step == n;
+          const uint32_t L = ks ? p.ks_len : p.len, pairs = (L + 1) / 2;
+          const uint32_t units = ks ? ks_units : br_units;
           if (!handed_over()) goto aux_done;  // the first pair's digits
           issue(0, 0);
           ++groups;
@@ -328,7 +337,8 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
       // Key stream: rows in consumption order (a blind-rotation step's digits of E.a and E.b; after the last
       // step the key switch's), a unit at a time into the next stage.
       const W *row = p.withhold ? nullptr : p.bsk;
-      uint32_t kd = 0, khalf = 0, kks = 0, kleft = n * 2 * p.len, kbatches = my_batches, kst = 0;
+      const uint32_t br_rows = (EXT ? 1 : n) * 2 * p.len;
+      uint32_t kd = 0, khalf = 0, kks = 0, kleft = br_rows, kbatches = my_batches, kst = 0;
       auto copy_keys = [&]() {
         if (!row || !kbatches) return;
         const uint32_t L = kks ? p.ks_len : p.len, ne = kd + 1 < L ? 2 : 1;
@@ -346,16 +356,16 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
         kleft -= ne;
         kd = kd + ne == L ? 0 : kd + ne;
         if (kleft == 0) {  // the next section: the key switch, or the next batch's rotation
-          kks ^= 1;
+          if (!EXT) kks ^= 1;
           row = kks ? p.ksk : p.bsk;
-          kleft = kks ? ks_chunks * p.ks_len : n * 2 * p.len;
+          kleft = kks ? ks_chunks * p.ks_len : br_rows;
           kbatches -= kks ^ 1;
         }
       };
       for (int s = 0; s < S; ++s) copy_keys();
       for (uint32_t b = 0; b < my_batches; ++b)
         for (uint32_t step = 0; step <= n; ++step) {
-          const uint32_t units = step == n ? ks_units : br_units;
+          const uint32_t units = !EXT && step == n ? ks_units : br_units;
           if (!handed_over()) goto key_done;
           if (b != 0 || step != 0) copy_keys();  // the stage of the last unit multiplied
           for (uint32_t u = 0; u <= units; ++u) {
@@ -390,10 +400,12 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
 
   for (uint32_t batch = blockIdx.x; batch < p.total_batches; batch += gridDim.x) {
     int jx = 0;
-    while (jx + 1 < p.njobs && p.jobs[jx + 1].first_batch <= batch) ++jx;
+    if constexpr (!EXT)
+      while (jx + 1 < p.njobs && p.jobs[jx + 1].first_batch <= batch) ++jx;
     const GateJob &job = p.jobs[jx];
-    const uint32_t gate = (batch - job.first_batch) * G + g;
-    const bool active = gate < job.count;
+    const unsigned long long item = (unsigned long long)batch * G + g;  // EXT
+    const uint32_t gate = EXT ? 0 : (batch - job.first_batch) * G + g;
+    const bool active = EXT ? item < ext.count : gate < job.count;
     const size_t lwe_words = (size_t)n + 1;
 
     // ---- input combine + modulus switch (as bootstrap_kernel) of coefficient k; absent gates rotate zeros
@@ -407,7 +419,7 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
       return (uint16_t)modswitch<F>(c, 2 * N);
     };
     // ---- ACC = (0, LUT * X^{-b}) (fhe_core/src/blind_rotation/rlwe/binary.rs:40-64) ----
-    {
+    if constexpr (!EXT) {
       const uint32_t bt = rotation(n);  // every thread of the group the same
       const int e = bt ? (int)(2 * N - bt) : 0;
       const W *lut = reinterpret_cast<const W *>(job.lut);
@@ -432,13 +444,14 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
 
     // ---- steps 0 .. n-1: blind rotation; step n: key switch ----
     for (uint32_t step = 0; step <= n; ++step) {
-      const bool ks = step == n, last = ks && batch + gridDim.x >= p.total_batches;
+      const bool ks = !EXT && step == n, last = step == n && batch + gridDim.x >= p.total_batches;
       const uint32_t L = ks ? p.ks_len : p.len, bits = ks ? p.ks_bits : p.bits;
       const uint32_t pairs = ks ? ks_pairs : br_pairs, units = ks ? ks_units : br_units;
-      if (step < n && step % Geo::MS_STEPS == 0) {  // the group's threads are past the rotations before
-        for (uint32_t k = t; k < Geo::MS_STEPS && step + k < n; k += 128) ms[k] = rotation(step + k);
-        sync();
-      }
+      if constexpr (!EXT)
+        if (step < n && step % Geo::MS_STEPS == 0) {  // the group's threads are past the rotations before
+          for (uint32_t k = t; k < Geo::MS_STEPS && step + k < n; k += 128) ms[k] = rotation(step + k);
+          sync();
+        }
       const uint32_t mask4 = ((1u << bits) - 1) * 0x01010101u;
       const int j0 = t & 15, jb = t >> 4;  // the thread's coefficients: 16 (8 jb + i) + j0
       // E of the part, 8 words a thread, kept in local memory (read back once per digit pair): registers
@@ -446,7 +459,11 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
       W e_mem[8];
       asm volatile("" ::"l"(e_mem) : "memory");
       auto load_part = [&](uint32_t prt) {
-        if (!ks) {
+        if constexpr (EXT) {
+          const W *y = ext.in + (item * 2 + prt) * N;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) e_mem[i] = active ? F::value(y[16 * (8 * jb + i) + j0]) : 0;
+        } else if (!ks) {
           // E = ACC * (X^r - 1) (lattice/src/rlwe.rs:437-487) in the reference's representation, then
           // canonical for the unsigned decomposition
           const int r = (int)ms[step % Geo::MS_STEPS];
@@ -632,7 +649,7 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
 
       // ---- inverse transforms and accumulator update (or extraction) ----
       W b0 = 0;
-      W *out = reinterpret_cast<W *>(job.out) + gate * lwe_words;
+      W *out = EXT ? ext.out + item * 2 * N : reinterpret_cast<W *>(job.out) + gate * lwe_words;
       if (ks) b0 = F::canon(F::add(acc_b[0], (W)(F::P >> 3)));  // evaluate.rs:52
       W sum[2][4], sum_b[2][4];  // of the a polynomial (h = 0), then the b polynomial
 #pragma unroll
@@ -663,7 +680,11 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
         sync();
         int ping = 0;
         NT::inverse(f, xbuf, ping, p.itw, t, sync);
-        if (!ks) {
+        if constexpr (EXT) {
+          if (active)
+#pragma unroll
+            for (int v = 0; v < V; ++v) out[h * N + NT::natural_pos(t, v)] = F::canon(f[v]);
+        } else if (!ks) {
           W *y = h == 0 ? acc_a : acc_b;
 #pragma unroll
           for (int v = 0; v < V; ++v) {

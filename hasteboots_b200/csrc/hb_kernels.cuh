@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(G * T, 1)
     ext_product_kernel(const typename F::W *__restrict__ rlwe_in, typename F::W *__restrict__ rlwe_out,
                        unsigned long long count, const typename F::W *__restrict__ rgsw,
                        uint32_t len, uint32_t bits, const typename F::W *__restrict__ tw_g,
-                       const typename F::W *__restrict__ itw_g, int *status, long long budget) {
+                       const typename F::W *__restrict__ itw_g, int *status, long long budget, uint32_t per_batch) {
   using W = typename F::W;
   using NT = GroupNtt<F, LOGN, T>;
   constexpr int N = 1 << LOGN, V = NT::V;
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(G * T, 1)
   W *xbuf = s_x + g * 2 * N;
   int ping = 0;
 
-  const unsigned long long batches = (count + G - 1) / G;
+  const unsigned long long batches = (count + per_batch - 1) / per_batch;  // per_batch <= G
   const unsigned long long my_batches =
       blockIdx.x < batches ? (batches - 1 - blockIdx.x) / gridDim.x + 1 : 0;
   const uint32_t cpb = 2 * len;
@@ -405,8 +405,8 @@ __global__ void __launch_bounds__(G * T, 1)
   const W off = F::acc_offset(2 * len);  // every slot sums 2 len products
 
   for (unsigned long long b = blockIdx.x; b < batches; b += gridDim.x) {
-    const unsigned long long item = b * G + g;
-    const bool active = item < count;
+    const unsigned long long item = b * per_batch + g;
+    const bool active = (uint32_t)g < per_batch && item < count;
     typename F::Acc acc_a[V], acc_b[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) {

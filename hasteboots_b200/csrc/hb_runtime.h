@@ -78,13 +78,16 @@ uint32_t ks_dim(const hb_params &p);
 // One persistent bootstrapping launch over a device job table (full grid, the keys' variant).
 int launch_set(hb_ctx *ctx, hb_keys *keys, int gates_per_cta, const hb::GateJob *djobs, int njobs,
                uint32_t batches, cudaStream_t stream);
-// The tensor-core form of the persistent kernel (hb_boot_tc.cu): its tables, built with the keys;
-// whether it covers a parameter set under a (T, G) variant; one launch over a device job table in place
+// The tensor-core form of the persistent kernel (hb_boot_tc.cu): its tables, built with the keys (where they
+// cannot be, or on a context that did not prepare the keys, the butterfly form serves); whether it covers a
+// parameter set under a (T, G) variant; one launch over a device job table in place
 // (status: another status word than the context's, or null).
-int tc_tables(hb_ctx *ctx, const hb_params &p);
-bool tc_applies(const hb_params &p, int T, int G);
+void tc_tables(hb_ctx *ctx, int field_id, uint32_t ring_dim);
+bool tc_applies(const hb_ctx *ctx, const hb_params &p, int T, int G);
 int launch_tc(hb_ctx *ctx, const hb_keys *keys, const hb::GateJob *djobs, int njobs, uint32_t batches, int *status,
               cudaStream_t stream);
+// External products over Goldilocks, N = 1024, bases up to 2^8, on a context with the tables.
+int launch_tc_ext(hb_ctx *ctx, const void *rgsw, uint32_t bits, uint32_t len, const void *in, void *out, size_t count);
 int launch_gates_per_cta(const hb_ctx *ctx, const hb_keys *keys, uint64_t gates);
 // The job record of `count` single-bootstrap gates (NAND..MAJORITY) of parameter set p.
 int gate_job(const hb_params &p, int gate, const void *c0, const void *c1, const void *c2, void *out,
