@@ -214,7 +214,13 @@ struct Mont32 {
   // x - P when x >= P, else x, as an unsigned minimum (x - P wraps above x when x < P): one add
   // and one min instead of a compare, a subtract and a select.
   HB_HD static W umin(W x, W y) { return y < x ? y : x; }
-  HB_HD static W canon(W x) { return umin(x, x - P); }
+  HB_HD static W canon(W x) {
+#ifdef __CUDA_ARCH__
+    return __viaddmin_u32(x, 0u - P, x);  // one instruction (7104 BABYBEAR gates, T = 64, G = 8: 146.5 -> 143.3 ms)
+#else
+    return umin(x, x - P);
+#endif
+  }
   // (t + m P) / 2^32 with m = -t P^-1 mod 2^32: t 2^-32 mod P, below 2P for t < P 2^32 (no final
   // subtraction).
   HB_HD static uint64_t redc_lazy(uint64_t t) {
@@ -233,7 +239,11 @@ struct Mont32 {
   // Canonical a - b: a - b, or a - b + P when it wrapped (then a - b + P < P <= the wrapped word).
   HB_HD static W sub(W a, W b) {
     const W d = a - b;
+#ifdef __CUDA_ARCH__
+    return __viaddmin_u32(d, P, d);
+#else
     return umin(d, d + P);
+#endif
   }
   HB_HD static W add_c(W a, W b) { return add(a, b); }
   HB_HD static W sub_c(W a, W b) { return sub(a, b); }
