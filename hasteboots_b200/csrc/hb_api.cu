@@ -60,6 +60,13 @@ int dev_alloc(hb_ctx *ctx, size_t bytes, void **out) {
   return HB_OK;
 }
 
+// The library's own constants and small tables, which a caller's HBM budget does not count.
+cudaError_t dev_constant(hb_ctx *ctx, size_t bytes, void **out) {
+  const cudaError_t e = cudaMalloc(out, bytes);
+  if (e == cudaSuccess) ctx->sizes.push_back({*out, 0});
+  return e;
+}
+
 void dev_free(hb_ctx *ctx, void *p) {
   if (!p) return;
   for (size_t i = 0; i < ctx->sizes.size(); ++i)
@@ -246,7 +253,7 @@ uint32_t ks_dim(const hb_params &p) {
 // half-CTA groups (words per thread: hb::dp_wide_words).
 int dp_tables(hb_ctx *ctx, const hb_params &p, int T) {
   if (p.ring_dim != 1024) return HB_OK;
-  tc_tables(ctx, p.field_id, p.ring_dim);
+  if (T == 128) tc_tables(ctx, p.field_id, p.ring_dim);
   const int ws = p.field_id == HB_FIELD_GOLDILOCKS ? 8 : 4;
   for (int cl = 0; cl < 2; ++cl) {
     // hb::dp_group_threads, hb::dp_groups: the groups' own transforms and the half-CTA groups'
@@ -817,6 +824,12 @@ int hb_ctx_create(int device, size_t hbm_budget, hb_ctx **out) {
   }
   ctx->d_status = (int *)st;
   cudaMemset(ctx->d_status, 0, sizeof(int) * 4);
+  // Room for the job table of any one gate call (run_rounds: two jobs, one of them cut in two): its second launch
+  // asks for no more of the budget than one launch did.
+  if (dev_constant(ctx, 4 * sizeof(GateJob), &ctx->jobs.ptr) == cudaSuccess)
+    ctx->jobs.cap = 4 * sizeof(GateJob);
+  else
+    cudaGetLastError();  // taken from the budget by the first call
   *out = ctx;
   return HB_OK;
 }

@@ -76,12 +76,13 @@ void tc_tables(hb_ctx *ctx, int field_id, uint32_t ring_dim) {
   if (tables(ctx, field_id, Geo::LOGN, &tb, 3)) return;
   const std::vector<unsigned char> t = build_tc(tb->psi);
   void *d = nullptr;
-  if (dev_alloc(ctx, t.size(), &d)) return;
-  if (cudaMemcpy(d, t.data(), t.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-    dev_free(ctx, d);
-    return;
-  }
-  ctx->tc_tables = d;
+  // without room for them the butterfly form runs; the error is not the caller's
+  cudaError_t e = dev_constant(ctx, t.size(), &d);
+  if (e == cudaSuccess) e = cudaMemcpy(d, t.data(), t.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess)
+    ctx->tc_tables = d;
+  else
+    cudaGetLastError();
 }
 
 bool tc_applies(const hb_ctx *ctx, const hb_params &p, int T, int G) {

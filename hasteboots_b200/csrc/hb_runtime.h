@@ -68,6 +68,7 @@ namespace hbrt {
 int fail(hb_ctx *ctx, int code, const char *fmt, ...);
 int cuda_fail(hb_ctx *ctx, cudaError_t e, const char *what);
 int dev_alloc(hb_ctx *ctx, size_t bytes, void **out);
+cudaError_t dev_constant(hb_ctx *ctx, size_t bytes, void **out);
 void dev_free(hb_ctx *ctx, void *p);
 int scratch(hb_ctx *ctx, Scratch &s, size_t bytes);
 int tables(hb_ctx *ctx, int field_id, uint32_t logn, DevTables **out, uint32_t logv = 4);

@@ -49,3 +49,28 @@ def test_rest_of_the_rounds(hb, ctx, set_id, tuned):
         assert (sk.decrypt(out) == np.where(bits[0, :count], bits[1, :count], bits[2, :count])).all()
     finally:
         ev.keys.free()
+
+
+@pytest.mark.parametrize("set_id", [0, 1])
+def test_device_calls_take_nothing_from_the_budget(hb, set_id):
+    """Once the keys are there a gate call, of one launch or of two, fits whatever the budget leaves."""
+    from gpu_util import empty_dev, from_dev, to_dev
+    from hasteboots_b200._lib import check, lib
+    sk = hb.KeyGen.generate_secret_key(hb_params_of(hb, set_id), 0)
+    ctx = hb.Context(0, hbm_budget=1 << 30)
+    ev = hb.Evaluator(sk, ctx)
+    try:
+        used = ctx.hbm_in_use()
+        bits = np.random.default_rng(5).integers(0, 2, (2, 1300)).astype(np.uint8)
+        c = [sk.encrypt(b, 5000 * i) for i, b in enumerate(bits)]
+        d = [to_dev(x) for x in c]
+        out = empty_dev(c[0].shape, c[0].dtype)
+        for count in (1, 149, 700, 1300):
+            check(lib().hb_gate_device(ctx.handle, ev.keys.handle, 0, d[0].data_ptr(), d[1].data_ptr(), None,
+                                       out.data_ptr(), count), "gate", ctx.handle)
+            ctx.synchronize()
+            assert ctx.hbm_in_use() == used, count
+        assert (sk.decrypt(from_dev(out, c[0].dtype)) == 1 - (bits[0] & bits[1])).all()
+    finally:
+        ev.keys.free()
+        ctx.close()
