@@ -618,8 +618,9 @@ __global__ void __launch_bounds__(G * T, 1) bootstrap_kernel(const BootParams<ty
     int jx = 0;
     while (jx + 1 < p.njobs && p.jobs[jx + 1].first_batch <= batch) ++jx;
     const GateJob &job = p.jobs[jx];
-    const uint32_t gate = (batch - job.first_batch) * job.per_batch + g;
-    const bool active = (uint32_t)g < job.per_batch && gate < job.count;
+    const uint32_t per_batch = G == 1 ? 1 : job.per_batch;
+    const uint32_t gate = (batch - job.first_batch) * per_batch + g;
+    const bool active = (uint32_t)g < per_batch && gate < job.count;
     const size_t lwe_words = (size_t)n + 1;
 
     // ---- input combine + modulus switch (Evaluator::nand etc., evaluate.rs:113-119) ----
