@@ -618,6 +618,7 @@ __global__ void __launch_bounds__(G * T, 1) bootstrap_kernel(const BootParams<ty
     int jx = 0;
     while (jx + 1 < p.njobs && p.jobs[jx + 1].first_batch <= batch) ++jx;
     const GateJob &job = p.jobs[jx];
+    // read from the table also at G = 1 a plain GOLDILOCKS gate took 0.4 % longer (25.65 -> 25.76 ms)
     const uint32_t per_batch = G == 1 ? 1 : job.per_batch;
     const uint32_t gate = (batch - job.first_batch) * per_batch + g;
     const bool active = (uint32_t)g < per_batch && gate < job.count;
