@@ -20,6 +20,7 @@
 // (BABYBEAR 12.8 against 12.4 ms), so it is built for Goldilocks only.
 #pragma once
 
+#include "hb_handover.h"
 #include "hb_kernels.cuh"
 #include "hb_tc.cuh"
 
@@ -277,16 +278,19 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
   // accumulators. Compute threads only arrive; the MMA and key warps wait, issue the MMAs, whose completion
   // (s_mma) is what the compute threads wait for, and refill the key stage that was multiplied. (From the
   // compute warps themselves the issue, which lasts as long as the MMAs run, held all others up: 5800
-  // cycles a unit.)
-  constexpr int kHandover = 5, kStop = 6, kHandoverThreads = Geo::THREADS + 64;
+  // cycles a unit.) Handovers take two named barriers in turn (hb_handover.h).
+  constexpr int kStop = 6, kHandoverThreads = Geo::THREADS + 64;
+  static_assert(kTcHandoverEven > G && kTcHandoverOdd > kStop && kTcHandoverEven < kStop, "named barriers overlap");
 
   if (warp >= kMmaWarp) {
     setmaxnreg_dec<Geo::AUX_REGS>();
-    auto handed_over = [&]() -> bool {
-      bar_sync<kHandover, kHandoverThreads>();
+    auto handed_over = [&](auto k) -> bool {  // handover k of the step, known up to its parity
+      bar_sync<tc_handover_barrier(decltype(k)::value), kHandoverThreads>();
       tc::fence_after();
       return *s_abort == 0;
     };
+    constexpr std::integral_constant<uint32_t, 0> even{};
+    constexpr std::integral_constant<uint32_t, 1> odd{};
     if (warp == kMmaWarp) {
       const uint64_t a1 = tc::smem_desc(smem_u32(s_a1), Geo::A1_LBO, 128), b1 = tc::smem_desc(smem_u32(s_b1), Geo::B1_LBO, 128);
       const uint64_t a2 = tc::smem_desc(smem_u32(s_a2), Geo::A2_LBO, 128), b2 = tc::smem_desc(smem_u32(s_b2), Geo::B2_LBO, 128);
@@ -316,18 +320,20 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
           const bool ks = !EXT && step == n;
           const uint32_t L = ks ? p.ks_len : p.len, pairs = (L + 1) / 2;
           const uint32_t units = ks ? ks_units : br_units;
-          if (!handed_over()) goto aux_done;  // the first pair's digits
+          if (!handed_over(even)) goto aux_done;  // the first pair's digits
           issue(0, 0);
           ++groups;
-          uint32_t pair = 0, half = 0;
-          for (uint32_t u = 0; u <= units; ++u) {
-            if (!handed_over()) goto aux_done;  // unit u twisted, unit u - 1 taken, unit u - 2 multiplied
-            if (u < units) {
-              issue(u + 1 < units ? half ^ 1 : 2, 2 * pair + 1 < L ? 2 : 1);
-              ++groups;
-            }
-            if (half == 1 && ++pair == pairs) pair = 0;
-            half ^= 1;
+          uint32_t pair = 0;
+          for (uint32_t u = 0;; u += 2) {  // units is even
+            if (!handed_over(odd)) goto aux_done;  // unit u twisted, unit u - 1 taken, unit u - 2 multiplied
+            if (u == units) break;
+            const uint32_t ne = 2 * pair + 1 < L ? 2 : 1;
+            issue(1, ne);
+            ++groups;
+            if (!handed_over(even)) goto aux_done;
+            issue(u + 2 < units ? 0 : 2, ne);
+            ++groups;
+            if (++pair == pairs) pair = 0;
           }
         }
     aux_done:
@@ -367,10 +373,13 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
       for (uint32_t b = 0; b < my_batches; ++b)
         for (uint32_t step = 0; step <= n; ++step) {
           const uint32_t units = !EXT && step == n ? ks_units : br_units;
-          if (!handed_over()) goto key_done;
+          if (!handed_over(even)) goto key_done;
           if (b != 0 || step != 0) copy_keys();  // the stage of the last unit multiplied
-          for (uint32_t u = 0; u <= units; ++u) {
-            if (!handed_over()) goto key_done;
+          for (uint32_t u = 0;; u += 2) {  // units is even
+            if (!handed_over(odd)) goto key_done;
+            if (u >= 2) copy_keys();
+            if (u == units) break;
+            if (!handed_over(even)) goto key_done;
             if (u >= 2) copy_keys();
           }
         }
@@ -389,11 +398,12 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
   uint32_t key_st = 0, key_par = 0;  // stage and phase of the key unit the next multiply takes
   uint32_t mma_par = 1;              // phase of the last MMA group handed over
   bool bad = false;                  // a wait of this thread ran out
-  bool stopped = false;              // the auxiliary warp still expects handovers
-  auto handover = [&]() {
+  bool stopped = false;              // the auxiliary warps still expect handovers
+  // Handover k of a step, k known up to its parity.
+  auto handover = [&](auto k) {
     tc::fence_async_smem();
     tc::fence_before();
-    bar_arrive<kHandover, kHandoverThreads>();
+    bar_arrive<tc_handover_barrier(decltype(k)::value), kHandoverThreads>();
   };
   // Barrier of the compute threads; true when a wait of some thread ran out. A thread whose wait ran out
   // goes on (later waits return at once) until the next of these.
@@ -614,7 +624,7 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
       // Units in a software pipeline: while the tensor core runs pass 1 of unit u and pass 2 of unit
       // u - 1, the threads multiply unit u - 2 with its keys; then they twist unit u and take unit u - 1.
       build_pair();
-      handover();
+      handover(std::integral_constant<uint32_t, 0>{});
       mma_par ^= 1;
       uint32_t pair = 0;  // unit u's pair in its part
       uint32_t ne0 = L > 1 ? 2 : 1, ne1 = 0, ne2 = 0;  // digits of units u, u - 1, u - 2
@@ -622,7 +632,8 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
         constexpr int half = decltype(half_c)::value;  // of units u and u - 2
         if (u >= 2) mac_unit(half_c, ne2);
         // Always waited for, whatever the launch's limit and after a key wait ran out too: a thread that ran
-        // ahead would arrive twice at one handover.
+        // ahead of the auxiliary warps would arrive twice at one handover (hb_handover.h). Nothing but the
+        // tensor core's own completion is waited for here.
         if (!mbar_wait_bounded(s_mma, mma_par, kDrainBudget) && !bad) {
           bad = true;
           atomicOr(p.status, STATUS_TIMEOUT);
@@ -631,7 +642,7 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
         if (u < units) twist_unit(half, ne0);
         if (u >= 1) take_unit(ne1);
         if (u + 1 < units && half == 1) build_pair();
-        handover();
+        handover(std::integral_constant<uint32_t, half + 1>{});
         if (u < units) mma_par ^= 1;
         ne2 = ne1;
         ne1 = ne0;
@@ -722,9 +733,9 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
   }
 
 aborted:
-  if (stopped) {  // the auxiliary warp stops at this handover
+  if (stopped) {  // the auxiliary warps stop at this handover, the first of a step that is not begun
     *s_abort = 1;
-    handover();
+    handover(std::integral_constant<uint32_t, 0>{});
   }
   tc::fence_before();
   __syncthreads();
