@@ -114,6 +114,7 @@ int launch_tc_ext(hb_ctx *ctx, const void *rgsw, uint32_t bits, uint32_t len, co
   prm.bits = bits;
   prm.status = ctx->d_status;
   prm.budget = wait_budget(ctx);
+  prm.withhold = ctx->withhold_keys;
   // at most 2^32 - 1 batches a launch
   for (size_t at = 0; at < count;) {
     const size_t part = std::min(count - at, (size_t)0xFFFFFF00u * Geo::G);
