@@ -198,8 +198,13 @@ int build_tables(hb_ctx *ctx, uint32_t logn, uint32_t logv, DevTables &t) {
     dev_free(ctx, dtw);
     return rc;
   }
-  cudaMemcpy(dtw, tw.data(), sizeof(Tw) * N, cudaMemcpyHostToDevice);
-  cudaMemcpy(ditw, itw.data(), sizeof(Tw) * N, cudaMemcpyHostToDevice);
+  cudaError_t e = upload(ctx, dtw, tw.data(), sizeof(Tw) * N);
+  if (e == cudaSuccess) e = upload(ctx, ditw, itw.data(), sizeof(Tw) * N);
+  if (e != cudaSuccess) {
+    dev_free(ctx, dtw);
+    dev_free(ctx, ditw);
+    return cuda_fail(ctx, e, "twiddle upload");
+  }
   t.tw = dtw;
   t.itw = ditw;
   return HB_OK;
@@ -817,13 +822,17 @@ int hb_ctx_create(int device, size_t hbm_budget, hb_ctx **out) {
     return HB_ERR_CUDA;
   }
   void *st = nullptr;
-  if (dev_alloc(ctx, sizeof(int) * 4, &st) != HB_OK) {
-    cudaStreamDestroy(ctx->stream);
-    delete ctx;
+  if (cudaStreamCreateWithFlags(&ctx->uploads, cudaStreamNonBlocking) != cudaSuccess ||
+      dev_alloc(ctx, sizeof(int) * 4, &st) != HB_OK) {
+    hb_ctx_destroy(ctx);
     return HB_ERR_CUDA;
   }
   ctx->d_status = (int *)st;
-  cudaMemset(ctx->d_status, 0, sizeof(int) * 4);
+  const int zero[4] = {0, 0, 0, 0};
+  if (upload(ctx, ctx->d_status, zero, sizeof(zero)) != cudaSuccess) {
+    hb_ctx_destroy(ctx);
+    return HB_ERR_CUDA;
+  }
   // Room for the job table of any one gate call (run_rounds: two jobs, one of them cut in two): its second launch
   // asks for no more of the budget than one launch did.
   if (dev_constant(ctx, 4 * sizeof(GateJob), &ctx->jobs.ptr) == cudaSuccess)
@@ -840,6 +849,7 @@ void hb_ctx_destroy(hb_ctx *ctx) {
   cudaStreamSynchronize(ctx->stream);
   for (auto &kv : ctx->sizes) cudaFree(kv.first);
   ctx->sizes.clear();
+  if (ctx->uploads) cudaStreamDestroy(ctx->uploads);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
 }
@@ -1796,10 +1806,10 @@ extern "C" int hb_batch_create(hb_ctx *ctx, const hb_job *jobs, size_t njobs, hb
     grp.grid = std::max(1u, std::min((unsigned)ctx->sms, bsum));
     rc = dev_alloc(ctx, sizeof(GateJob) * tab.size(), &grp.djobs);
     if (!rc) {
-      cudaMemcpy(grp.djobs, tab.data(), sizeof(GateJob) * tab.size(), cudaMemcpyHostToDevice);
-      if (cudaStreamCreateWithFlags(&grp.stream, cudaStreamNonBlocking) != cudaSuccess ||
+      if (upload(ctx, grp.djobs, tab.data(), sizeof(GateJob) * tab.size()) != cudaSuccess ||
+          cudaStreamCreateWithFlags(&grp.stream, cudaStreamNonBlocking) != cudaSuccess ||
           cudaEventCreateWithFlags(&grp.done, cudaEventDisableTiming) != cudaSuccess)
-        rc = fail(ctx, HB_ERR_CUDA, "stream creation");
+        rc = fail(ctx, HB_ERR_CUDA, "job table upload and stream creation");
     }
     b->groups.push_back(grp);
   }

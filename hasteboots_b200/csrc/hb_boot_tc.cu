@@ -78,7 +78,7 @@ void tc_tables(hb_ctx *ctx, int field_id, uint32_t ring_dim) {
   void *d = nullptr;
   // without room for them the butterfly form runs; the error is not the caller's
   cudaError_t e = dev_constant(ctx, t.size(), &d);
-  if (e == cudaSuccess) e = cudaMemcpy(d, t.data(), t.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && (e = upload(ctx, d, t.data(), t.size())) != cudaSuccess) dev_free(ctx, d);
   if (e == cudaSuccess)
     ctx->tc_tables = d;
   else

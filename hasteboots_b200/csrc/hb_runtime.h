@@ -35,6 +35,7 @@ struct hb_ctx {
   int device = 0;
   int sms = 148;
   cudaStream_t stream = nullptr;
+  cudaStream_t uploads = nullptr;  // copies of tables (hbrt::upload)
   int *d_status = nullptr;
   size_t budget = 0;
   size_t in_use = 0;
@@ -69,6 +70,13 @@ int fail(hb_ctx *ctx, int code, const char *fmt, ...);
 int cuda_fail(hb_ctx *ctx, cudaError_t e, const char *what);
 int dev_alloc(hb_ctx *ctx, size_t bytes, void **out);
 cudaError_t dev_constant(hb_ctx *ctx, size_t bytes, void **out);
+// Host words to the device, there for every stream when this returns and not waiting for the context's work. (A
+// copy on the legacy stream from pageable memory may return once the words are staged, and the library's streams
+// are not ordered behind that stream.)
+inline cudaError_t upload(const hb_ctx *ctx, void *dst, const void *src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->uploads);
+  return e == cudaSuccess ? cudaStreamSynchronize(ctx->uploads) : e;
+}
 void dev_free(hb_ctx *ctx, void *p);
 int scratch(hb_ctx *ctx, Scratch &s, size_t bytes);
 int tables(hb_ctx *ctx, int field_id, uint32_t logn, DevTables **out, uint32_t logv = 4);
