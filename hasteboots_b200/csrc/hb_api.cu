@@ -788,7 +788,8 @@ int default_threads_per_gate(const hb_params &p) {
   if (env && (atoi(env) == 64 || atoi(env) == 128)) return atoi(env);
   // measured best tiles on B200; a ternary key's second set of sums makes 16 words a thread too many (700
   // CUSTOM_TERNARY gates 29.1 ms at 64 threads, 24.6 at 128)
-  return p.field_id == HB_FIELD_GOLDILOCKS || p.lwe_ternary ? 128 : 64;
+  // (N = 1024: other dimensions have no bootstrapping kernel, and their uploads stay refused)
+  return p.field_id == HB_FIELD_GOLDILOCKS || (p.lwe_ternary && p.ring_dim == 1024) ? 128 : 64;
 }
 
 int default_gates_per_cta(int field_id) {
