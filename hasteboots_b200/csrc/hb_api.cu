@@ -786,10 +786,14 @@ size_t word_size(const hb_params &p) { return p.field_id == HB_FIELD_GOLDILOCKS 
 int default_threads_per_gate(const hb_params &p) {
   const char *env = getenv("HB_THREADS_PER_GATE");
   if (env && (atoi(env) == 64 || atoi(env) == 128)) return atoi(env);
-  // measured best tiles on B200; a ternary key's second set of sums makes 16 words a thread too many (700
-  // CUSTOM_TERNARY gates 29.1 ms at 64 threads, 24.6 at 128)
-  // (N = 1024: other dimensions have no bootstrapping kernel, and their uploads stay refused)
-  return p.field_id == HB_FIELD_GOLDILOCKS || (p.lwe_ternary && p.ring_dim == 1024) ? 128 : 64;
+  if (p.field_id == HB_FIELD_GOLDILOCKS) return 128;  // measured best tiles on B200
+  // A ternary key's second set of sums makes 16 words a thread too many, and four inverse transforms a step are
+  // shorter with 8; but each digit's transform has one exchange less with 16. ms at 64 / 128 threads, by digits:
+  // 592 gates n = 512: 2 13.0 / 9.5, 4 (CUSTOM_TERNARY) 16.3 / 14.8, 6 21.2 / 20.1, 7 23.6 / 22.7, 9 28.2 / 28.0;
+  // n = 1024: 4 31.0 / 30.1, 5 35.6 / 35.5, 6 40.1 / 40.9, 7 44.0 / 46.4, 9 (DEFAULT_TERNARY) 53.6 / 57.2. 296 gates
+  // favour 128 throughout (DEFAULT_TERNARY 45.8 / 43.8), one gate 64 from four digits on (5.3 / 5.4 and 19.5 / 21.8).
+  // (N = 1024: other dimensions have no bootstrapping kernel, and their uploads stay refused.)
+  return p.lwe_ternary && p.br_len <= 6 && p.ring_dim == 1024 ? 128 : 64;
 }
 
 int default_gates_per_cta(int field_id) {

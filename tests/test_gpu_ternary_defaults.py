@@ -35,3 +35,23 @@ def test_a_dimension_without_kernels_stays_refused(hb, ctx):
     rc = lib().hb_keys_upload(ctx.handle, ctypes.byref(raw), bsk.ctypes.data_as(ctypes.c_void_p),
                               ksk.ctypes.data_as(ctypes.c_void_p), ctypes.byref(keys))
     assert rc == HB_ERR_UNSUPPORTED and not keys.value
+
+
+@pytest.mark.parametrize("words,threads", [(dict(), 64), (dict(br_bits=5, br_len=6), 128),
+                                           (dict(br_bits=4, br_len=7), 64), (dict(br_bits=14, br_len=2), 128)])
+def test_default_group_size_follows_the_digits(hb, ctx, words, threads):
+    """DEFAULT_TERNARY with its nine digits, and around the rule's line. Gates under both layouts give the same words."""
+    from hasteboots_b200._lib import check, lib
+    sk = hb.KeyGen.generate_secret_key(hb.Parameters(ternary(hb, 3, lwe_dim=60, **words), "ternary"), 0)
+    ev = hb.Evaluator(sk, ctx)
+    try:
+        t, g = ctypes.c_int(), ctypes.c_int()
+        lib().hb_keys_config(ev.keys.handle, ctypes.byref(t), ctypes.byref(g))
+        assert (t.value, g.value) == (threads, 4)
+        bits = np.random.default_rng(3).integers(0, 2, (2, 200)).astype(np.uint8)
+        c = [sk.encrypt(b, 1000 * i) for i, b in enumerate(bits)]
+        out = ev.nand(*c)
+        check(lib().hb_keys_set_config(ctx.handle, ev.keys.handle, 192 - threads, 4), "config", ctx.handle)
+        assert (ev.nand(*c) == out).all()
+    finally:
+        ev.keys.free()
