@@ -778,14 +778,6 @@ __global__ void __launch_bounds__(G * T, 1) bootstrap_kernel(const BootParams<ty
         const W *k0 = pipe.acquire();
         const W *k1 = pipe.acquire_next();
         if (active) {
-          if (F::FOLD < (1 << 20) && nprod + 2 > (uint32_t)F::FOLD) {
-            nprod = 0;
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-              F::acc_fold(acc_x[v]);
-              F::acc_fold(acc_y[v]);
-            }
-          }
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             F::acc_mac2(acc_x[v], x[v], k0[v * T + t], y[v], k1[v * T + t]);
@@ -818,7 +810,7 @@ __global__ void __launch_bounds__(G * T, 1) bootstrap_kernel(const BootParams<ty
             trace_digit(y, j + 1);
             NT::forward_small2(x, y, xbuf, ping, s_tw, t, sync);
           }
-          if constexpr (!TERN) {
+          if constexpr (!TERN && !F::WIDE) {
             if (!mac_pair(x, y)) goto aborted;
           } else {
             if (!mac_digit(x) || !mac_digit(y)) goto aborted;
