@@ -730,7 +730,9 @@ int run_rounds(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> jobs) {
   cut_front(keys->p, jobs, batch_sum(jobs, tuned) / sms * sms, tuned, table);
   uint64_t rest = 0;
   for (auto &j : jobs) rest += j.count;
-  uint64_t even = (rest + sms - 1) / sms;  // gates per SM of the rest, in at most one batch per SM
+  // Gates per SM of the rest, in at most one batch per SM: fewer than one batch per SM of the tuned variant are
+  // left (none at all on one SM), so this ends at `tuned` at the latest.
+  uint64_t even = (rest + sms - 1) / sms;
   while (rest && batch_sum(jobs, even) > sms) ++even;
   // The tensor-core form lasts its four gates whether they are there or not; and one gate short of a full CTA
   // does not pay in the other form (its idle group polls for keys: 900 BABYBEAR gates seven to a CTA 24.7 ms,
@@ -743,7 +745,9 @@ int run_rounds(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> jobs) {
     if (even > 1)
       for (int g : variants(keys->p, keys->threads_per_gate))
         if ((uint64_t)g >= even && g < rest_variant) rest_variant = g;
-    if (even + 1 >= (uint64_t)rest_variant) even = rest_variant;
+    // (the tensor-core form takes whole batches only)
+    if (even + 1 >= (uint64_t)rest_variant || tc_applies(ctx, keys->p, keys->threads_per_gate, rest_variant))
+      even = rest_variant;
     cut_front(keys->p, jobs, ~0ull / tuned, (uint32_t)even, table);
   }
   if (table.empty()) return HB_OK;

@@ -192,7 +192,8 @@ struct TcAcc {
     cross(m01, m2, y1, l0);
     merge(m01, m2);
   }
-  // e0 .. e3 reduced, minus e4 2^32 (2^128 = -2^32 mod Q; e4 < 2^32 / 2^32 products)
+  // e0 .. e3 reduced, minus e4 2^32 (2^128 = -2^32 mod Q). e4 counts carries, at most one per direct and per
+  // merge: below 2^32 - 1 for any number of digits, as e4 2^32 < Q needs.
   __device__ __forceinline__ uint64_t value() const {
     return glx::sub_c(glx::reduce_canon((uint32_t)e01, (uint32_t)(e01 >> 32), (uint32_t)e23, (uint32_t)(e23 >> 32)),
                       (uint64_t)e4 << 32);
@@ -633,7 +634,7 @@ __global__ void __launch_bounds__(TcGeo::THREADS + TcGeo::AUX, 1)
         if (u >= 2) mac_unit(half_c, ne2);
         // Always waited for, whatever the launch's limit and after a key wait ran out too: a thread that ran
         // ahead of the auxiliary warps would arrive twice at one handover (hb_handover.h). Nothing but the
-        // tensor core's own completion is waited for here.
+        // tensor core's own completion is waited for here, about 2 s a unit if it never came.
         if (!mbar_wait_bounded(s_mma, mma_par, kDrainBudget) && !bad) {
           bad = true;
           atomicOr(p.status, STATUS_TIMEOUT);

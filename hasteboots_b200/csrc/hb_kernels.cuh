@@ -71,7 +71,8 @@ struct GateJob {
   int32_t s0, s1, s2;
   uint32_t count;
   uint32_t first_batch;
-  uint32_t per_batch;  // gates per batch, at most the kernel's G (bootstrap_kernel; the other forms: fixed)
+  uint32_t per_batch;  // gates per batch: at most the kernel's G (bootstrap_kernel), exactly four
+                       // (bootstrap_tc_kernel, which does not read it), one (bootstrap_dp_kernel, the same)
 };
 
 // Ring of S shared-memory stages fed by the TMA unit with consecutive 2N-word chunks of key
