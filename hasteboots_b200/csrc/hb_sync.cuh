@@ -62,6 +62,10 @@ template <int ID, int THREADS>
 __device__ __forceinline__ void bar_sync() {
   asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory");
 }
+template <int THREADS>
+__device__ __forceinline__ void bar_sync(int id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(THREADS) : "memory");
+}
 template <int ID, int THREADS>
 __device__ __forceinline__ bool bar_or(bool x) {
   uint32_t r;
