@@ -613,10 +613,9 @@ int run_jobs(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> &jobs, bool plain,
   uint64_t gates = 0;
   for (auto &j : jobs) gates += j.count;
   if (!plain && !trace) return run_rounds(ctx, keys, jobs);
-  const int G = plain ? 1 : launch_gates_per_cta(ctx, keys, gates), T = keys->threads_per_gate,
-            fld = keys->p.field_id;
+  const int T = keys->threads_per_gate, fld = keys->p.field_id;
   const bool tern = keys->p.lwe_ternary != 0, ksc = ks_dim(keys->p) < keys->p.ring_dim;
-  if (trace && (plain || G != 1 || tern || gates != 1))
+  if (trace && (plain || tern || gates != 1))
     return fail(ctx, HB_ERR_UNSUPPORTED, "accumulator traces are recorded for one gate under a binary LWE key");
   for (auto &j : jobs) j.per_batch = 1;
 #define HB_CASE(FLD, TT, GG, TN, KC)                                             \
@@ -624,7 +623,7 @@ int run_jobs(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> &jobs, bool plain,
     return launch_boot<FLD, 10, TT, TN, KC>(ctx, keys, jobs, plain, trace);
   HB_BOOT_VARIANTS(HB_CASE)
 #undef HB_CASE
-  return fail(ctx, HB_ERR_UNSUPPORTED, "no compiled kernel with %d threads per gate and %d gates per CTA", T, G);
+  return fail(ctx, HB_ERR_UNSUPPORTED, "no compiled kernel with %d threads per gate and one gate per CTA", T);
 }
 
 // Gates-per-CTA variants compiled for a parameter set and group size (the autotuner's candidates).
@@ -638,15 +637,16 @@ std::vector<int> variants(const hb_params &p, int T) {
   return v;
 }
 
-uint32_t batches_of(const std::vector<GateJob> &jobs, int G) {
-  uint32_t b = 0;
-  for (auto &j : jobs) b += (j.count + G - 1) / G;
-  return b;
+hb::LaunchShape shape_of(const hb_ctx *ctx, const hb_keys *keys, const std::vector<GateJob> &jobs, int tuned, bool latency) {
+  std::vector<uint32_t> counts;
+  for (auto &j : jobs) counts.push_back(j.count);
+  return hb::launch_shape(counts, (uint64_t)std::max(1, ctx->sms), tuned, variants(keys->p, keys->threads_per_gate),
+                          keys->threads_per_gate, tc_applies(ctx, keys->p, keys->threads_per_gate, tuned), latency);
 }
 
 // One batched persistent launch over a device job table that is already in place.
 template <class F, int LOGN, int T, int G, bool TERN, bool KSC>
-int launch_table(hb_ctx *ctx, hb_keys *keys, const GateJob *djobs, int njobs, uint32_t batches,
+int launch_table(hb_ctx *ctx, hb_keys *keys, bool tensor, const GateJob *djobs, int njobs, uint32_t batches,
                  unsigned grid, cudaStream_t stream) {
   using W = typename F::W;
   constexpr int N = 1 << LOGN;
@@ -654,7 +654,7 @@ int launch_table(hb_ctx *ctx, hb_keys *keys, const GateJob *djobs, int njobs, ui
   int rc = tables(ctx, F::FIELD_ID, LOGN, &tb, hb::GroupNtt<F, LOGN, T>::LOGV);
   if (rc) return rc;
   if constexpr (T == 128 && G == 4 && !TERN) {
-    if (tc_applies(ctx, keys->p, T, G)) {
+    if (tensor) {
       rc = launch_tc(ctx, keys, djobs, njobs, batches, nullptr, stream);
       if (!rc) ctx->launches += 1;
       return rc;
@@ -679,13 +679,14 @@ int launch_table(hb_ctx *ctx, hb_keys *keys, const GateJob *djobs, int njobs, ui
   return HB_OK;
 }
 
-int launch_table_any(hb_ctx *ctx, hb_keys *keys, int G, const GateJob *djobs, int njobs,
+// tensor: the tensor-core form, where tc_applies.
+int launch_table_any(hb_ctx *ctx, hb_keys *keys, int G, bool tensor, const GateJob *djobs, int njobs,
                      uint32_t batches, unsigned grid, cudaStream_t stream) {
   const int T = keys->threads_per_gate, fld = keys->p.field_id;
   const bool tern = keys->p.lwe_ternary != 0, ksc = ks_dim(keys->p) < keys->p.ring_dim;
 #define HB_CASE(FLD, TT, GG, TN, KC)                                             \
   if (fld == field_of<FLD>() && T == TT && G == GG && tern == TN && ksc == KC) \
-    return launch_table<FLD, 10, TT, GG, TN, KC>(ctx, keys, djobs, njobs, batches, grid, stream);
+    return launch_table<FLD, 10, TT, GG, TN, KC>(ctx, keys, tensor, djobs, njobs, batches, grid, stream);
   HB_BOOT_VARIANTS(HB_CASE)
 #undef HB_CASE
   return fail(ctx, HB_ERR_UNSUPPORTED, "no compiled kernel with %d threads per gate and %d gates per CTA", T, G);
@@ -725,6 +726,7 @@ uint64_t batch_sum(const std::vector<GateJob> &jobs, uint64_t per) {
 // gates 48.2 -> 29.3 ms, 2500 BABYBEAR 72.3 -> 53.8, 600 GOLDILOCKS 92.4 -> 56.4.)
 int run_rounds(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> jobs) {
   const uint32_t tuned = (uint32_t)keys->gates_per_cta;
+  const bool tensor = tc_applies(ctx, keys->p, keys->threads_per_gate, (int)tuned);
   const uint64_t sms = (uint64_t)std::max(1, ctx->sms);
   std::vector<GateJob> table;
   cut_front(keys->p, jobs, batch_sum(jobs, tuned) / sms * sms, tuned, table);
@@ -737,7 +739,7 @@ int run_rounds(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> jobs) {
   // The tensor-core form lasts its four gates whether they are there or not; and one gate short of a full CTA
   // does not pay in the other form (its idle group polls for keys: 900 BABYBEAR gates seven to a CTA 24.7 ms,
   // eight 24.2).
-  if (even > 1 && (even + 1 >= tuned || tc_applies(ctx, keys->p, keys->threads_per_gate, (int)tuned)))
+  if (even > 1 && (even + 1 >= tuned || tensor))
     cut_front(keys->p, jobs, ~0ull / tuned, tuned, table);
   const size_t first = table.size();
   int rest_variant = even <= 1 ? 1 : (int)tuned;
@@ -745,9 +747,7 @@ int run_rounds(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> jobs) {
     if (even > 1)
       for (int g : variants(keys->p, keys->threads_per_gate))
         if ((uint64_t)g >= even && g < rest_variant) rest_variant = g;
-    // (the tensor-core form takes whole batches only)
-    if (even + 1 >= (uint64_t)rest_variant || tc_applies(ctx, keys->p, keys->threads_per_gate, rest_variant))
-      even = rest_variant;
+    if (even + 1 >= (uint64_t)rest_variant) even = rest_variant;
     cut_front(keys->p, jobs, ~0ull / tuned, (uint32_t)even, table);
   }
   if (table.empty()) return HB_OK;
@@ -765,9 +765,9 @@ int run_rounds(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> jobs) {
   if (e != cudaSuccess) return cuda_fail(ctx, e, "job table upload");
   const GateJob *djobs = (const GateJob *)ctx->jobs.ptr;
   if (batches[0])
-    rc = launch_table_any(ctx, keys, tuned, djobs, (int)first, batches[0], (unsigned)ctx->sms, ctx->stream);
+    rc = launch_table_any(ctx, keys, tuned, tensor, djobs, (int)first, batches[0], (unsigned)ctx->sms, ctx->stream);
   if (!rc && batches[1])
-    rc = launch_table_any(ctx, keys, rest_variant, djobs + first, (int)(table.size() - first), batches[1],
+    rc = launch_table_any(ctx, keys, rest_variant, false, djobs + first, (int)(table.size() - first), batches[1],
                           (unsigned)ctx->sms, ctx->stream);
   return rc;
 }
@@ -1476,20 +1476,20 @@ int noalloc_address(hb_ctx *ctx, unsigned char **out) {
   return HB_OK;
 }
 
-// Gates per CTA of the allocation-free MUX: the keys' variant, or, when that is the one-gate
-// latency variant (which the batched launches here do not use), the smallest compiled G > 1 for
-// the keys' group size.
-int noalloc_gates_per_cta(const hb_keys *keys) {
-  if (keys->gates_per_cta > 1) return keys->gates_per_cta;
-  std::vector<int> v = variants(keys->p, keys->threads_per_gate);
-  return v.empty() ? 0 : *std::min_element(v.begin(), v.end());
+// The shape of a layer of the allocation-free MUX: batched launches only. Keys tuned to the one-gate form take the
+// smallest batched variant of their group size.
+hb::LaunchShape batched_shape(const hb_ctx *ctx, const hb_keys *keys, const std::vector<GateJob> &jobs) {
+  const std::vector<int> v = variants(keys->p, keys->threads_per_gate);
+  if (v.empty()) return {0, false};
+  const int tuned = keys->gates_per_cta > 1 ? keys->gates_per_cta : *std::min_element(v.begin(), v.end());
+  return shape_of(ctx, keys, jobs, tuned, false);
 }
 
 template <class F, int LOGN, int T, int G, bool TERN, bool KSC>
-int launch_noalloc(hb_ctx *ctx, hb_keys *keys, const DevTables *tb, const GateJob *djobs, int njobs,
+int launch_noalloc(hb_ctx *ctx, hb_keys *keys, bool tensor, const DevTables *tb, const GateJob *djobs, int njobs,
                    uint32_t batches, int *dstatus) {
   if constexpr (T == 128 && G == 4 && !TERN)
-    if (tc_applies(ctx, keys->p, T, G)) return launch_tc(ctx, keys, djobs, njobs, batches, dstatus, ctx->stream);
+    if (tensor) return launch_tc(ctx, keys, djobs, njobs, batches, dstatus, ctx->stream);
   using W = typename F::W;
   constexpr int N = 1 << LOGN;
   hb::BootParams<W> prm{};
@@ -1510,12 +1510,12 @@ int launch_noalloc(hb_ctx *ctx, hb_keys *keys, const DevTables *tb, const GateJo
 }
 
 int noalloc_layer(hb_ctx *ctx, hb_keys *keys, const DevTables *tb, const GateJob *djobs, int njobs,
-                  uint32_t batches, int *dstatus, int G) {
-  const int T = keys->threads_per_gate, fld = keys->p.field_id;
+                  uint32_t batches, int *dstatus, hb::LaunchShape shape) {
+  const int T = keys->threads_per_gate, G = shape.gates_per_cta, fld = keys->p.field_id;
   const bool tern = keys->p.lwe_ternary != 0, ksc = ks_dim(keys->p) < keys->p.ring_dim;
 #define HB_CASE(FLD, TT, GG, TN, KC)                                                       \
   if (fld == field_of<FLD>() && T == TT && G == GG && GG > 1 && tern == TN && ksc == KC) \
-    return launch_noalloc<FLD, 10, TT, GG, TN, KC>(ctx, keys, tb, djobs, njobs, batches, dstatus);
+    return launch_noalloc<FLD, 10, TT, GG, TN, KC>(ctx, keys, shape.tensor, tb, djobs, njobs, batches, dstatus);
   HB_BOOT_VARIANTS(HB_CASE)
 #undef HB_CASE
   return fail(ctx, HB_ERR_UNSUPPORTED, "no compiled kernel with %d gates per CTA", G);
@@ -1552,8 +1552,6 @@ extern "C" int hb_gate_mux_device_noalloc(hb_ctx *ctx, hb_keys *keys, const void
 
   // MUX (tfhe/src/bfhe/evaluate.rs:245-262): t0 = and(c0, c1), t1 = and(not c0, c2) in one launch,
   // then out = bootstrap(t0 + t1, or) in a second.
-  const int G = noalloc_gates_per_cta(keys);
-  if (G <= 1) return fail(ctx, HB_ERR_UNSUPPORTED, "no batched kernel compiled for these keys");
   GateJob jobs[3];
   jobs[0] = make_job(P, HB_GATE_AND, p.ring_dim, c0, c1, nullptr, t0, (uint32_t)count);
   jobs[1] = jobs[0];
@@ -1562,11 +1560,15 @@ extern "C" int hb_gate_mux_device_noalloc(hb_ctx *ctx, hb_keys *keys, const void
   jobs[1].s0 = -1;  // not(c0) = -c0 + Q/4 on the body
   jobs[1].add_b = P >> 2;
   jobs[2] = make_job(P, HB_GATE_MUX, p.ring_dim, t0, t1, nullptr, out, (uint32_t)count);
-  const uint32_t per_job = (uint32_t)((count + G - 1) / G);
-  jobs[0].first_batch = 0;
-  jobs[1].first_batch = per_job;
-  jobs[2].first_batch = 0;
-  for (GateJob &j : jobs) j.per_batch = (uint32_t)G;
+  hb::LaunchShape shape[2];
+  uint32_t batches[2];
+  for (int layer = 0; layer < 2; ++layer) {
+    std::vector<GateJob> l(jobs + 2 * layer, jobs + 2 + layer);
+    shape[layer] = batched_shape(ctx, keys, l);
+    if (shape[layer].gates_per_cta <= 1) return fail(ctx, HB_ERR_UNSUPPORTED, "no batched kernel compiled for these keys");
+    batches[layer] = lay_out(l, shape[layer].gates_per_cta);
+    std::copy(l.begin(), l.end(), jobs + 2 * layer);
+  }
 
   // The array keeps the previous call's contents: the status word must start at zero.
   e = cudaMemsetAsync(dstatus, 0, sizeof(int), ctx->stream);
@@ -1576,8 +1578,7 @@ extern "C" int hb_gate_mux_device_noalloc(hb_ctx *ctx, hb_keys *keys, const void
   // The second layer reads t0 and t1, so it runs only when the first one finished all its waits.
   int h = 0;
   for (int layer = 0; layer < 2; ++layer) {
-    rc = layer == 0 ? noalloc_layer(ctx, keys, tb, djobs, 2, 2 * per_job, dstatus, G)
-                    : noalloc_layer(ctx, keys, tb, djobs + 2, 1, per_job, dstatus, G);
+    rc = noalloc_layer(ctx, keys, tb, djobs + 2 * layer, 2 - layer, batches[layer], dstatus, shape[layer]);
     if (rc) return rc;
     e = cudaMemcpyAsync(&h, dstatus, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -1695,14 +1696,13 @@ extern "C" int hb_autotune(hb_ctx *ctx, hb_keys *keys, uint32_t sample_gates, in
     if (rc) break;
     std::vector<GateJob> jobs{make_job(modulus_of(keys->p.field_id), HB_GATE_NAND, 1024, buf, buf,
                                        nullptr, (char *)buf + bytes, sample_gates)};
-    jobs[0].first_batch = 0;
-    jobs[0].per_batch = (uint32_t)G;
-    const uint32_t batches = batches_of(jobs, G);
+    const uint32_t batches = lay_out(jobs, G);
     cudaMemcpyAsync(tab, jobs.data(), sizeof(GateJob), cudaMemcpyHostToDevice, ctx->stream);
     float best_ms = 1e30f;
     for (int rep = 0; rep < 3 && !rc; ++rep) {  // rep 0 warms up
       cudaEventRecord(e0, ctx->stream);
-      rc = launch_table_any(ctx, keys, G, (const GateJob *)tab, 1, batches, ctx->sms, ctx->stream);
+      rc = launch_table_any(ctx, keys, G, tc_applies(ctx, keys->p, T, G), (const GateJob *)tab, 1, batches, ctx->sms,
+                            ctx->stream);
       cudaEventRecord(e1, ctx->stream);
       if (cudaEventSynchronize(e1) != cudaSuccess) rc = cuda_fail(ctx, cudaGetLastError(), "autotune");
       float ms = 0;
@@ -1739,7 +1739,7 @@ struct hb_batch {
     int njobs = 0;
     uint32_t batches = 0;
     unsigned grid = 0;
-    int gates_per_cta = 0;
+    hb::LaunchShape shape{};
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
   };
@@ -1800,19 +1800,10 @@ extern "C" int hb_batch_create(hb_ctx *ctx, const hb_job *jobs, size_t njobs, hb
     hb_batch::Group grp;
     grp.keys = keysets[k];
     auto &tab = tables_h[k];
-    uint64_t set_gates = 0;
-    for (auto &t : tab) set_gates += t.count;
-    const int G = launch_gates_per_cta(ctx, grp.keys, set_gates);
-    grp.gates_per_cta = G;
-    uint32_t bsum = 0;
-    for (auto &t : tab) {
-      t.first_batch = bsum;
-      t.per_batch = (uint32_t)G;
-      bsum += (t.count + G - 1) / G;
-    }
-    grp.batches = bsum;
+    grp.shape = launch_shape(ctx, grp.keys, tab);
+    grp.batches = lay_out(tab, grp.shape.gates_per_cta);
     grp.njobs = (int)tab.size();
-    grp.grid = std::max(1u, std::min((unsigned)ctx->sms, bsum));
+    grp.grid = std::max(1u, std::min((unsigned)ctx->sms, grp.batches));
     rc = dev_alloc(ctx, sizeof(GateJob) * tab.size(), &grp.djobs);
     if (!rc) {
       if (upload(ctx, grp.djobs, tab.data(), sizeof(GateJob) * tab.size()) != cudaSuccess ||
@@ -1832,8 +1823,8 @@ extern "C" int hb_batch_create(hb_ctx *ctx, const hb_job *jobs, size_t njobs, hb
       if (e != cudaSuccess || rc) break;
       e = cudaStreamWaitEvent(grp.stream, b->fork, 0);
       if (e == cudaSuccess)
-        rc = launch_table_any(ctx, grp.keys, grp.gates_per_cta, (const GateJob *)grp.djobs, grp.njobs,
-                              grp.batches, grp.grid, grp.stream);
+        rc = launch_table_any(ctx, grp.keys, grp.shape.gates_per_cta, grp.shape.tensor, (const GateJob *)grp.djobs,
+                              grp.njobs, grp.batches, grp.grid, grp.stream);
       if (e == cudaSuccess && !rc) e = cudaEventRecord(grp.done, grp.stream);
       if (e == cudaSuccess && !rc) e = cudaStreamWaitEvent(ctx->stream, grp.done, 0);
     }
@@ -1876,29 +1867,24 @@ extern "C" int hb_batch_info(const hb_batch *b, uint64_t *gates, int *launches, 
 
 namespace hbrt {
 
-int launch_set(hb_ctx *ctx, hb_keys *keys, int G, const GateJob *djobs, int njobs, uint32_t batches,
+int launch_set(hb_ctx *ctx, hb_keys *keys, hb::LaunchShape shape, const GateJob *djobs, int njobs, uint32_t batches,
                cudaStream_t stream) {
-  return launch_table_any(ctx, keys, G, djobs, njobs, batches, (unsigned)ctx->sms, stream);
+  return launch_table_any(ctx, keys, shape.gates_per_cta, shape.tensor, djobs, njobs, batches, (unsigned)ctx->sms, stream);
 }
 
-// Gates per CTA for one launch of `gates` gates: the keys' autotuned (throughput) choice, unless that
-// leaves SMs idle; then the smallest compiled variant that still gives every CTA an SM of its own,
-// so that fewer gates share an SM and a small launch finishes sooner.
-int launch_gates_per_cta(const hb_ctx *ctx, const hb_keys *keys, uint64_t gates) {
-  const int tuned = keys->gates_per_cta;
-  const uint64_t sms = (uint64_t)std::max(1, ctx->sms);
-  if (gates >= sms * (uint64_t)tuned) return tuned;
-  std::vector<int> cand = variants(keys->p, keys->threads_per_gate);
-  cand.push_back(1);
-  std::sort(cand.begin(), cand.end());
-  for (int g : cand) {
-    // The tensor-core form fills the smaller batched variants' place: a launch lasts one CTA's four gates
-    // whether they are there or not (GOLDILOCKS 46 ms), less than three gates in the other form (56 ms) and
-    // more than one in the latency form (18 ms).
-    if (g > 1 && g != tuned && tc_applies(ctx, keys->p, keys->threads_per_gate, tuned)) continue;
-    if (g <= tuned && (gates + g - 1) / g <= sms) return g;
+hb::LaunchShape launch_shape(const hb_ctx *ctx, const hb_keys *keys, const std::vector<GateJob> &jobs) {
+  return shape_of(ctx, keys, jobs, keys->gates_per_cta, true);
+}
+
+// Jobs end to end in batches of G gates; batches do not span jobs.
+uint32_t lay_out(std::vector<GateJob> &jobs, int G) {
+  uint32_t b = 0;
+  for (auto &j : jobs) {
+    j.first_batch = b;
+    j.per_batch = (uint32_t)G;
+    b += (j.count + G - 1) / G;
   }
-  return tuned;
+  return b;
 }
 
 int gate_job(const hb_params &p, int gate, const void *c0, const void *c1, const void *c2, void *out,

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/hb_gpu.h"
+#include "hb_shape.h"
 
 namespace hb {
 struct GateJob;
@@ -84,8 +85,11 @@ int check_status(hb_ctx *ctx);
 long long wait_budget(const hb_ctx *ctx);
 // The key switch's dimension n' = next_pow2(n) (fhe_core/src/key_switch/rlwe.rs:40-43).
 uint32_t ks_dim(const hb_params &p);
-// One persistent bootstrapping launch over a device job table (full grid, the keys' variant).
-int launch_set(hb_ctx *ctx, hb_keys *keys, int gates_per_cta, const hb::GateJob *djobs, int njobs,
+// A launch of a key set's jobs: its shape (hb_shape.h), the jobs laid out in its batches (their number), and one
+// persistent bootstrapping launch over the job table on the device.
+hb::LaunchShape launch_shape(const hb_ctx *ctx, const hb_keys *keys, const std::vector<hb::GateJob> &jobs);
+uint32_t lay_out(std::vector<hb::GateJob> &jobs, int gates_per_cta);
+int launch_set(hb_ctx *ctx, hb_keys *keys, hb::LaunchShape shape, const hb::GateJob *djobs, int njobs,
                uint32_t batches, cudaStream_t stream);
 // The tensor-core form of the persistent kernel (hb_boot_tc.cu): its tables, built with the keys (where they
 // cannot be, or on a context that did not prepare the keys, the butterfly form serves); whether it covers a
@@ -97,7 +101,6 @@ int launch_tc(hb_ctx *ctx, const hb_keys *keys, const hb::GateJob *djobs, int nj
               cudaStream_t stream);
 // External products over Goldilocks, N = 1024, bases up to 2^8, on a context with the tables.
 int launch_tc_ext(hb_ctx *ctx, const void *rgsw, uint32_t bits, uint32_t len, const void *in, void *out, size_t count);
-int launch_gates_per_cta(const hb_ctx *ctx, const hb_keys *keys, uint64_t gates);
 // The job record of `count` single-bootstrap gates (NAND..MAJORITY) of parameter set p.
 int gate_job(const hb_params &p, int gate, const void *c0, const void *c1, const void *c2, void *out,
              uint32_t count, hb::GateJob *job);

@@ -175,15 +175,8 @@ int launch_wave(hb_server *s, std::vector<Request *> reqs, int slot) {
   std::vector<cudaEvent_t> joins;
   int rc = HB_OK;
   for (size_t k = 0; k < sets.size() && !rc; ++k) {
-    uint64_t set_gates = 0;
-    for (auto &j : tabs[k]) set_gates += j.count;
-    const int G = hbrt::launch_gates_per_cta(ctx, sets[k], set_gates);
-    uint32_t batches = 0;
-    for (auto &j : tabs[k]) {
-      j.first_batch = batches;
-      j.per_batch = (uint32_t)G;
-      batches += (j.count + G - 1) / G;
-    }
+    const hb::LaunchShape shape = hbrt::launch_shape(ctx, sets[k], tabs[k]);
+    const uint32_t batches = hbrt::lay_out(tabs[k], shape.gates_per_cta);
     cudaStream_t st = s->set_streams[slot * kMaxSets + k];
     void *dtab = nullptr;
     cudaStreamWaitEvent(st, fork, 0);
@@ -195,7 +188,7 @@ int launch_wave(hb_server *s, std::vector<Request *> reqs, int slot) {
       break;
     }
     w.tables.push_back(dtab);
-    rc = hbrt::launch_set(ctx, sets[k], G, (const hb::GateJob *)dtab, (int)tabs[k].size(), batches, st);
+    rc = hbrt::launch_set(ctx, sets[k], shape, (const hb::GateJob *)dtab, (int)tabs[k].size(), batches, st);
     cudaEvent_t j;
     cudaEventCreateWithFlags(&j, cudaEventDisableTiming);
     cudaEventRecord(j, st);

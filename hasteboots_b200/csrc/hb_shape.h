@@ -1,0 +1,73 @@
+// hb_shape.h -- the shape of one launch over a list of jobs (a batch, a serving wave, a layer of the allocation-free
+// MUX): gates per CTA, and the butterfly or the tensor-core form. Batches of a launch do not span jobs, so jobs of
+// a few gates leave every batch short.
+#pragma once
+
+#include <algorithm>
+#include <cstdint>
+#include <vector>
+
+namespace hb {
+
+struct LaunchShape {
+  int gates_per_cta;
+  bool tensor;
+};
+
+// How long a batch holds its CTA by the gates in it, in halves of what one more gate adds. Measured on B200, ms of a
+// batch of 1, 2, 3, 4 gates in the butterfly form with 128 threads a gate: GOLDILOCKS 28.7, 38.3, 50.0, 63.7, ZAMA 43.2,
+// 58.5, 76.5, 97.5; the tensor-core form lasts its four gates whether they are there or not: 45.8 and 69.5. With 64
+// threads (two warps) a gate, two gates last as long as one: 2, 4, 6, 8 of DEFAULT_TERNARY 26.4, 32.2, 43.9, 57.0, BABYBEAR
+// 12.1, 15.4, 19.9, 23.7, CUSTOM_TERNARY 7.4, 9.0, 12.5, 15.4.
+constexpr uint32_t kTensorBatch = 8;
+inline uint32_t batch_lasts(uint32_t gates, int threads_per_gate, bool tensor) {
+  if (tensor) return kTensorBatch;
+  return threads_per_gate >= 128 ? 2 * gates + 3 : (gates + 1) / 2 * 4 + 4;
+}
+
+// The launch's longest CTA: CTA i of sms takes batches i, i + sms, ...
+inline uint64_t launch_lasts(const std::vector<uint32_t> &counts, uint64_t sms, int gates_per_cta, int threads_per_gate,
+                             bool tensor) {
+  std::vector<uint64_t> cta(sms, 0);
+  uint64_t at = 0;
+  for (uint32_t c : counts)
+    while (c) {
+      const uint32_t b = std::min<uint32_t>(c, (uint32_t)gates_per_cta);
+      cta[at] += batch_lasts(b, threads_per_gate, tensor);
+      at = at + 1 == sms ? 0 : at + 1;
+      c -= b;
+    }
+  return *std::max_element(cta.begin(), cta.end());
+}
+
+// tuned: the keys' variant; variants: the batched ones compiled for them and their group size; tensor: whether the
+// tensor-core form covers the keys under `tuned`; latency: whether the one-gate form may be taken.
+//
+// One gate per CTA while every gate gets an SM of its own; else the tensor-core form or the variant, up to the tuned
+// one, that is over first, the smallest of those that last the same (absent groups of a larger CTA poll for keys).
+// What one shape for all job lists cost: 300 GOLDILOCKS jobs of one gate 87 ms in the butterfly form, 137 in the
+// tensor-core form, of three gates 150 and 137; 40 DEFAULT_TERNARY jobs of 30 gates 87 ms six per CTA, 113 eight.
+inline LaunchShape launch_shape(const std::vector<uint32_t> &counts, uint64_t sms, int tuned, std::vector<int> variants,
+                                int threads_per_gate, bool tensor, bool latency) {
+  uint64_t gates = 0;
+  for (uint32_t c : counts) gates += c;
+  if (tuned <= 1 || (latency && gates <= sms)) return {1, false};
+  std::sort(variants.begin(), variants.end());
+  LaunchShape best{tuned, false};
+  uint64_t shortest = ~0ull;
+  if (tensor) {
+    best.tensor = true;
+    shortest = launch_lasts(counts, sms, tuned, threads_per_gate, true);
+  }
+  for (int g : variants) {
+    if (g > tuned) break;
+    const uint64_t lasts = launch_lasts(counts, sms, g, threads_per_gate, false);
+    if (lasts < shortest) {
+      shortest = lasts;
+      best = {g, false};
+    }
+  }
+  return best;
+}
+
+}  // namespace hb
