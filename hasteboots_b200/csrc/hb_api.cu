@@ -1200,15 +1200,9 @@ int hb_external_product_device(hb_ctx *ctx, int field_id, uint32_t log_n, uint32
   cudaSetDevice(ctx->device);
   if (field_id == HB_FIELD_GOLDILOCKS) {
     if (log_n == 10) {
-      // The tensor-core form (digits of a byte) lasts four RLWEs per SM whether they are there or not, so whole
-      // rounds of four go to it and a rest of more than two; a rest of one or two per SM is shorter in the
-      // butterfly form. l = 13, B = 2^5 on B200, butterfly / tensor form: 148 RLWEs 66 / 98 us, 296 93 / 99,
-      // 444 122 / 99, 592 153 / 100, 4096 994 / 677.
       size_t rest = count;
       if (bits <= 8 && ctx->tc_tables) {
-        const size_t sms = (size_t)ctx->sms;
-        rest = count % (4 * sms);
-        if (rest > 2 * sms) rest = 0;
+        rest = hb::external_products_by_butterflies(count, len, (size_t)ctx->sms);
         if (count > rest) {
           const int rc = launch_tc_ext(ctx, d_rgsw, bits, len, rlwe_in, rlwe_out, count - rest);
           if (rc || rest == 0) return rc;

@@ -1,9 +1,10 @@
-// hb_shape.h -- the shape of one launch over a list of jobs (a batch, a serving wave, a layer of the allocation-free
-// MUX): gates per CTA, and the butterfly or the tensor-core form. Batches of a launch do not span jobs, so jobs of
-// a few gates leave every batch short.
+// hb_shape.h -- the shapes of launches. Of one over a list of jobs (a batch, a serving wave, a layer of the
+// allocation-free MUX): gates per CTA, and the butterfly or the tensor-core form; batches of a launch do not span
+// jobs, so jobs of a few gates leave every batch short. Of a batch of external products: which form takes which.
 #pragma once
 
 #include <algorithm>
+#include <cstddef>
 #include <cstdint>
 #include <vector>
 
@@ -68,6 +69,22 @@ inline LaunchShape launch_shape(const std::vector<uint32_t> &counts, uint64_t sm
     }
   }
   return best;
+}
+
+// External products over Goldilocks, N = 1024, digits of a byte: how many of the last RLWEs the butterfly form takes,
+// the tensor-core form the whole rounds of four per SM before them. The latter lasts four RLWEs per SM whether they
+// are there or not, so a rest of more than two per SM goes to it and a smaller one is shorter in the butterfly form.
+// l = 13, B = 2^5 on B200, butterfly / tensor form: 148 RLWEs 66 / 98 us, 296 93 / 99, 444 122 / 99, 592 153 / 100, 4096
+// 994 / 677. With few digits it saves little or nothing a round (592 RLWEs, l = 1, 2, 3: 25.1 / 29.6, 35.3 / 33.2, 45.5 /
+// 41.4), and the rest's launch of its own costs more than a CTA's last one or two RLWEs in the butterfly form alone
+// (593: 33.3 / 46.8, 47.5 / 53.7, 60.4 / 65.9; l = 4: 74.2 / 74.1), for two digits after five rounds also more than
+// any batch of its (2964: 184.5 / 190.9).
+inline size_t external_products_by_butterflies(size_t count, uint32_t len, size_t sms) {
+  const size_t round = 4 * sms;
+  size_t rest = count % round;
+  if (rest > 2 * sms) rest = 0;
+  const bool tail_pays = len > 3 || rest == 0 || (rest > 2 && (len == 3 || count < 5 * round));
+  return len > 1 && tail_pays ? rest : count;
 }
 
 }  // namespace hb

@@ -1,7 +1,8 @@
 """The shape of a launch over a list of jobs (hasteboots_b200/csrc/hb_shape.h), whose batches do not span jobs, against
 the measured times of a batch. Over GOLDILOCKS no list of jobs may take longer than in the butterfly form alone (the
 tensor-core form lasts four gates whether they are there or not, so launches of jobs of one or two gates must not
-go to it); over the 32-bit fields none longer than in the best of the compiled variants."""
+go to it); over the 32-bit fields none longer than in the best of the compiled variants. And external products over
+GOLDILOCKS, by digits and number of RLWEs."""
 
 import os
 import random
@@ -22,8 +23,13 @@ BABYBEAR = {1: 12.0, 2: 12.1, 3: 15.3, 4: 15.4, 5: 19.6, 6: 19.9, 7: 23.7, 8: 23
 
 DRIVER = r"""
 #include <cstdio>
+#include <cstdlib>
 #include "hb_shape.h"
-int main() {
+int main(int argc, char **argv) {
+  if (argc == 4) {
+    printf("%zu\n", hb::external_products_by_butterflies(strtoull(argv[1], 0, 10), (uint32_t)atoi(argv[2]), strtoull(argv[3], 0, 10)));
+    return 0;
+  }
   unsigned sms, threads, tuned, nv, tensor, latency, n;
   while (scanf("%u %u %u %u %u %u", &sms, &threads, &tuned, &tensor, &latency, &nv) == 6) {
     std::vector<int> v(nv);
@@ -39,11 +45,16 @@ int main() {
 
 
 @pytest.fixture(scope="module")
-def shape():
+def exe():
     d = tempfile.mkdtemp()
     src, exe = os.path.join(d, "s.cpp"), os.path.join(d, "s")
     open(src, "w").write(DRIVER)
     subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-O1", "-I", CSRC, src, "-o", exe], check=True)
+    return exe
+
+
+@pytest.fixture(scope="module")
+def shape(exe):
 
     def run(lists, threads, tuned, variants, tensor=False, latency=True, sms=SMS):
         text = "".join("%d %d %d %d %d %d %s\n%d %s\n" % (sms, threads, tuned, tensor, latency, len(variants),
@@ -106,3 +117,30 @@ def test_edges(shape):
     # variants beyond the tuned one are not taken, in any order
     assert shape([[5000]], 64, 6, [8, 6, 4]) == [(6, False)]
     assert shape([[5000], [2]], 64, 6, [6, 4], sms=1) == [(6, False), (4, False)]
+
+
+# us of one call on B200 by digits and RLWEs: all in the butterfly form, and the whole rounds in the tensor-core form
+# with a rest of at most two per SM in a launch of its own
+EXTERNAL = {
+    1: {592: (25.1, 29.6), 593: (33.3, 46.8), 740: (45.6, 46.7), 1184: (45.5, 53.7), 1185: (53.6, 70.0), 4096: (164, 199)},
+    2: {592: (35.3, 33.2), 593: (47.7, 53.6), 594: (51.5, 53.5), 596: (63.7, 53.5), 740: (64.0, 53.7), 888: (64.1, 57.7),
+        1184: (64.2, 59.8), 1185: (77.4, 80.1), 1188: (92.5, 80.1), 2369: (137, 149), 2372: (152.5, 148.1),
+        2961: (170, 191), 2964: (184.5, 190.9), 3553: (204, 226), 4096: (237, 218), 4148: (247, 256), 8192: (469, 426)},
+    3: {592: (45.5, 41.4), 593: (61.7, 65.8), 594: (66.0, 65.8), 596: (82.3, 65.8), 888: (87.7, 70.1), 1188: (121.5, 100.9),
+        2369: (181, 187), 2372: (202, 187), 2961: (226, 239), 2964: (244, 238), 3556: (285, 281), 4096: (315, 279)},
+    4: {592: (53.9, 43.6), 593: (74.2, 74.1), 740: (107, 73.7), 1185: (123, 111), 2369: (224, 202), 4096: (389, 298)},
+    13: {592: (153, 100), 593: (214, 180), 700: (302, 179), 1184: (312, 213), 4096: (1012, 693)},
+}
+
+
+@pytest.mark.parametrize("digits", sorted(EXTERNAL))
+def test_form_of_external_products(exe, digits):
+    def rest(count):
+        return int(subprocess.run([exe, str(count), str(digits), str(SMS)], capture_output=True, text=True, check=True).stdout)
+    for count, (butterfly, tensor) in EXTERNAL[digits].items():
+        assert (butterfly if rest(count) == count else tensor) <= 1.01 * min(butterfly, tensor), count
+    for count in (1, 2, 148, 296, 297, 592, 593, 888, 889, 1184, 100000):
+        r, whole = rest(count), 4 * SMS
+        assert r == count or r <= 2 * SMS and ((count - r) % whole == 0 or r == 0)
+        if digits >= 4:
+            assert r == (count % whole if count % whole <= 2 * SMS else 0)
