@@ -1005,8 +1005,9 @@ __device__ __forceinline__ const W *cluster_peer(const W *p, uint32_t rank) {
 //
 // KST: every thread copies its key words of a digit into shared memory (cp.async) before the
 // digit's transform and waits for them after it; otherwise the key words are read from global
-// memory after the transform. No L2 prefetch: with the row's own words prefetched before the transform one
-// GOLDILOCKS gate measured 10.06 ms, with the next step's row 11.9, without 9.93 (ZAMA 13.70, 17.5, 13.63).
+// memory after the transform. 64-bit keys laid out for 64 threads: with an L2 prefetch of the row's own words before
+// the transform (one GOLDILOCKS gate 11.67 ms, 12.01 without; ZAMA 15.63 and 16.33); for 128 threads without (10.06
+// with it, 9.93 without, with the next step's row 11.9; ZAMA 13.70, 13.63, 17.5).
 //
 // C > 1: a cluster of C CTAs (C SMs) per gate. The digits go to the C * D groups of the cluster;
 // each CTA sums its groups' partials, the CTAs read each other's sums through distributed shared
@@ -1182,6 +1183,12 @@ __global__ void __launch_bounds__(D * T, 1) bootstrap_dp_kernel(const BootParams
             cp_async_word(kbuf + N + v * T + t, krow + N + kbase + v * KT);
           }
           cp_async_commit();
+        } else if constexpr (sizeof(W) == 8 && KT == 64) {
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(krow + kbase + v * KT));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(krow + N + kbase + v * KT));
+          }
         }
         W x[V];
         if (KSC && ks) {
