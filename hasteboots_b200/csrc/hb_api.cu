@@ -637,11 +637,12 @@ std::vector<int> variants(const hb_params &p, int T) {
   return v;
 }
 
-hb::LaunchShape shape_of(const hb_ctx *ctx, const hb_keys *keys, const std::vector<GateJob> &jobs, int tuned, bool latency) {
+hb::LaunchShape shape_of(const hb_ctx *ctx, const hb_keys *keys, const std::vector<GateJob> &jobs, int tuned,
+                         bool latency, bool shared) {
   std::vector<uint32_t> counts;
   for (auto &j : jobs) counts.push_back(j.count);
   return hb::launch_shape(counts, (uint64_t)std::max(1, ctx->sms), tuned, variants(keys->p, keys->threads_per_gate),
-                          keys->threads_per_gate, tc_applies(ctx, keys->p, keys->threads_per_gate, tuned), latency);
+                          keys->threads_per_gate, tc_applies(ctx, keys->p, keys->threads_per_gate, tuned), latency, shared);
 }
 
 // One batched persistent launch over a device job table that is already in place.
@@ -1476,7 +1477,7 @@ hb::LaunchShape batched_shape(const hb_ctx *ctx, const hb_keys *keys, const std:
   const std::vector<int> v = variants(keys->p, keys->threads_per_gate);
   if (v.empty()) return {0, false};
   const int tuned = keys->gates_per_cta > 1 ? keys->gates_per_cta : *std::min_element(v.begin(), v.end());
-  return shape_of(ctx, keys, jobs, tuned, false);
+  return shape_of(ctx, keys, jobs, tuned, false, false);
 }
 
 template <class F, int LOGN, int T, int G, bool TERN, bool KSC>
@@ -1794,7 +1795,7 @@ extern "C" int hb_batch_create(hb_ctx *ctx, const hb_job *jobs, size_t njobs, hb
     hb_batch::Group grp;
     grp.keys = keysets[k];
     auto &tab = tables_h[k];
-    grp.shape = launch_shape(ctx, grp.keys, tab);
+    grp.shape = launch_shape(ctx, grp.keys, tab, keysets.size() > 1);
     grp.batches = lay_out(tab, grp.shape.gates_per_cta);
     grp.njobs = (int)tab.size();
     grp.grid = std::max(1u, std::min((unsigned)ctx->sms, grp.batches));
@@ -1866,8 +1867,8 @@ int launch_set(hb_ctx *ctx, hb_keys *keys, hb::LaunchShape shape, const GateJob 
   return launch_table_any(ctx, keys, shape.gates_per_cta, shape.tensor, djobs, njobs, batches, (unsigned)ctx->sms, stream);
 }
 
-hb::LaunchShape launch_shape(const hb_ctx *ctx, const hb_keys *keys, const std::vector<GateJob> &jobs) {
-  return shape_of(ctx, keys, jobs, keys->gates_per_cta, true);
+hb::LaunchShape launch_shape(const hb_ctx *ctx, const hb_keys *keys, const std::vector<GateJob> &jobs, bool shared) {
+  return shape_of(ctx, keys, jobs, keys->gates_per_cta, true, shared);
 }
 
 // Jobs end to end in batches of G gates; batches do not span jobs.

@@ -85,9 +85,9 @@ int check_status(hb_ctx *ctx);
 long long wait_budget(const hb_ctx *ctx);
 // The key switch's dimension n' = next_pow2(n) (fhe_core/src/key_switch/rlwe.rs:40-43).
 uint32_t ks_dim(const hb_params &p);
-// A launch of a key set's jobs: its shape (hb_shape.h), the jobs laid out in its batches (their number), and one
+// A launch of a key set's jobs: its shape (hb_shape.h; shared: among other launches), the jobs laid out in its batches (their number), and one
 // persistent bootstrapping launch over the job table on the device.
-hb::LaunchShape launch_shape(const hb_ctx *ctx, const hb_keys *keys, const std::vector<hb::GateJob> &jobs);
+hb::LaunchShape launch_shape(const hb_ctx *ctx, const hb_keys *keys, const std::vector<hb::GateJob> &jobs, bool shared);
 uint32_t lay_out(std::vector<hb::GateJob> &jobs, int gates_per_cta);
 int launch_set(hb_ctx *ctx, hb_keys *keys, hb::LaunchShape shape, const hb::GateJob *djobs, int njobs,
                uint32_t batches, cudaStream_t stream);

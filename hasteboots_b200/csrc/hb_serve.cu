@@ -175,7 +175,7 @@ int launch_wave(hb_server *s, std::vector<Request *> reqs, int slot) {
   std::vector<cudaEvent_t> joins;
   int rc = HB_OK;
   for (size_t k = 0; k < sets.size() && !rc; ++k) {
-    const hb::LaunchShape shape = hbrt::launch_shape(ctx, sets[k], tabs[k]);
+    const hb::LaunchShape shape = hbrt::launch_shape(ctx, sets[k], tabs[k], sets.size() > 1 || !s->inflight.empty());
     const uint32_t batches = hbrt::lay_out(tabs[k], shape.gates_per_cta);
     cudaStream_t st = s->set_streams[slot * kMaxSets + k];
     void *dtab = nullptr;

@@ -26,43 +26,56 @@ inline uint32_t batch_lasts(uint32_t gates, int threads_per_gate, bool tensor) {
   return threads_per_gate >= 128 ? 2 * gates + 3 : (gates + 1) / 2 * 4 + 4;
 }
 
-// The launch's longest CTA: CTA i of sms takes batches i, i + sms, ...
-inline uint64_t launch_lasts(const std::vector<uint32_t> &counts, uint64_t sms, int gates_per_cta, int threads_per_gate,
-                             bool tensor) {
+// How long a launch of its own lasts, its longest CTA (CTA i of sms takes batches i, i + sms, ...), and how long it holds
+// SMs in all.
+struct LaunchLasts {
+  uint64_t longest, total;
+};
+inline LaunchLasts launch_lasts(const std::vector<uint32_t> &counts, uint64_t sms, int gates_per_cta, int threads_per_gate,
+                                bool tensor) {
   std::vector<uint64_t> cta(sms, 0);
-  uint64_t at = 0;
+  uint64_t at = 0, total = 0;
   for (uint32_t c : counts)
     while (c) {
-      const uint32_t b = std::min<uint32_t>(c, (uint32_t)gates_per_cta);
-      cta[at] += batch_lasts(b, threads_per_gate, tensor);
+      const uint32_t b = std::min<uint32_t>(c, (uint32_t)gates_per_cta), lasts = batch_lasts(b, threads_per_gate, tensor);
+      cta[at] += lasts;
+      total += lasts;
       at = at + 1 == sms ? 0 : at + 1;
       c -= b;
     }
-  return *std::max_element(cta.begin(), cta.end());
+  return {*std::max_element(cta.begin(), cta.end()), total};
 }
 
 // tuned: the keys' variant; variants: the batched ones compiled for them and their group size; tensor: whether the
-// tensor-core form covers the keys under `tuned`; latency: whether the one-gate form may be taken.
+// tensor-core form covers the keys under `tuned`; latency: whether the one-gate form may be taken; shared: whether
+// other launches (of other key sets, of the wave before) take the SMs that this one leaves.
 //
-// One gate per CTA while every gate gets an SM of its own; else the tensor-core form or the variant, up to the tuned
-// one, that is over first, the smallest of those that last the same (absent groups of a larger CTA poll for keys).
-// What one shape for all job lists cost: 300 GOLDILOCKS jobs of one gate 87 ms in the butterfly form, 137 in the
-// tensor-core form, of three gates 150 and 137; 40 DEFAULT_TERNARY jobs of 30 gates 87 ms six per CTA, 113 eight.
+// One gate per CTA while every gate gets an SM of its own. Else a launch of its own takes the tensor-core form or the
+// variant, up to the tuned one, that is over first, the smallest of those that last the same (absent groups of a larger
+// CTA poll for keys). What one shape for all job lists cost: 300 GOLDILOCKS jobs of one gate 87 ms in the butterfly
+// form, 137 in the tensor-core form, of three gates 150 and 137; 40 DEFAULT_TERNARY jobs of 30 gates 87 ms six per CTA,
+// 113 eight. Among other launches it takes the form that holds SMs for less, and the smallest variant whose CTAs, were
+// they full, got an SM each (24 jobs of BABYBEAR, GOLDILOCKS and ZAMA in one graph: 277 ms, 282 with the BABYBEAR
+// launch of 1179 gates cut in sixes, its shortest alone).
 inline LaunchShape launch_shape(const std::vector<uint32_t> &counts, uint64_t sms, int tuned, std::vector<int> variants,
-                                int threads_per_gate, bool tensor, bool latency) {
+                                int threads_per_gate, bool tensor, bool latency, bool shared) {
   uint64_t gates = 0;
   for (uint32_t c : counts) gates += c;
   if (tuned <= 1 || (latency && gates <= sms)) return {1, false};
   std::sort(variants.begin(), variants.end());
-  LaunchShape best{tuned, false};
-  uint64_t shortest = ~0ull;
-  if (tensor) {
-    best.tensor = true;
-    shortest = launch_lasts(counts, sms, tuned, threads_per_gate, true);
+  LaunchLasts tc{~0ull, ~0ull};
+  if (tensor) tc = launch_lasts(counts, sms, tuned, threads_per_gate, true);
+  if (shared) {
+    if (tensor && tc.total <= launch_lasts(counts, sms, tuned, threads_per_gate, false).total) return {tuned, true};
+    for (int g : variants)
+      if (g <= tuned && (gates + (uint64_t)g - 1) / (uint64_t)g <= sms) return {g, false};
+    return {tuned, false};
   }
+  LaunchShape best{tuned, tensor};
+  uint64_t shortest = tc.longest;
   for (int g : variants) {
     if (g > tuned) break;
-    const uint64_t lasts = launch_lasts(counts, sms, g, threads_per_gate, false);
+    const uint64_t lasts = launch_lasts(counts, sms, g, threads_per_gate, false).longest;
     if (lasts < shortest) {
       shortest = lasts;
       best = {g, false};

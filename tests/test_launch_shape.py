@@ -30,14 +30,14 @@ int main(int argc, char **argv) {
     printf("%zu\n", hb::external_products_by_butterflies(strtoull(argv[1], 0, 10), (uint32_t)atoi(argv[2]), strtoull(argv[3], 0, 10)));
     return 0;
   }
-  unsigned sms, threads, tuned, nv, tensor, latency, n;
-  while (scanf("%u %u %u %u %u %u", &sms, &threads, &tuned, &tensor, &latency, &nv) == 6) {
+  unsigned sms, threads, tuned, nv, tensor, latency, shared, n;
+  while (scanf("%u %u %u %u %u %u %u", &sms, &threads, &tuned, &tensor, &latency, &shared, &nv) == 7) {
     std::vector<int> v(nv);
     for (int &x : v) if (scanf("%d", &x) != 1) return 1;
     if (scanf("%u", &n) != 1) return 1;
     std::vector<uint32_t> c(n);
     for (uint32_t &x : c) if (scanf("%u", &x) != 1) return 1;
-    const hb::LaunchShape s = hb::launch_shape(c, sms, (int)tuned, v, (int)threads, tensor != 0, latency != 0);
+    const hb::LaunchShape s = hb::launch_shape(c, sms, (int)tuned, v, (int)threads, tensor != 0, latency != 0, shared != 0);
     printf("%d %d\n", s.gates_per_cta, (int)s.tensor);
   }
 }
@@ -56,8 +56,8 @@ def exe():
 @pytest.fixture(scope="module")
 def shape(exe):
 
-    def run(lists, threads, tuned, variants, tensor=False, latency=True, sms=SMS):
-        text = "".join("%d %d %d %d %d %d %s\n%d %s\n" % (sms, threads, tuned, tensor, latency, len(variants),
+    def run(lists, threads, tuned, variants, tensor=False, latency=True, sms=SMS, shared=False):
+        text = "".join("%d %d %d %d %d %d %d %s\n%d %s\n" % (sms, threads, tuned, tensor, latency, shared, len(variants),
                                                          " ".join(map(str, variants)), len(c), " ".join(map(str, c)))
                        for c in lists)
         out = subprocess.run([exe], input=text, capture_output=True, text=True, check=True).stdout.split()
@@ -108,6 +108,25 @@ def test_variant_of_the_32_bit_fields(shape, batch, variants):
     for counts, (g, tensor) in zip(lists, shape(lists, 64, variants[-1], variants, False, False)):
         assert not tensor
         assert ms(counts, g, batch) <= 1.10 * min(ms(counts, v, batch) for v in variants), (g, counts[:9], len(counts))
+
+
+def total(counts, g, batch):
+    return sum(batch[min(g, c - at)] for c in counts for at in range(0, c, g))
+
+
+def test_among_other_launches(shape):
+    """The form that holds SMs for less, and gates per CTA from the number of gates alone."""
+    lists = job_lists()
+    tensor_batch = dict.fromkeys(GOLDILOCKS, TENSOR)
+    for counts, (g, tensor) in zip(lists, shape(lists, 128, 4, [3, 4], True, shared=True)):
+        if sum(counts) > SMS:
+            best = min(total(counts, 4, GOLDILOCKS), total(counts, 4, tensor_batch))
+            assert total(counts, g, tensor_batch if tensor else GOLDILOCKS) <= 1.10 * best
+    baby = [24, 10, 278, 463, 44, 2, 8, 350]
+    assert shape([baby], 64, 8, [4, 6, 8], shared=True) == [(8, False)]
+    assert total(baby, 8, BABYBEAR) < total(baby, 6, BABYBEAR)
+    lists = [[148], [200], [592], [600], [888], [1184], [1185], [1] * 300]
+    assert [g for g, _ in shape(lists, 64, 8, [4, 6, 8], shared=True)] == [1, 4, 4, 6, 6, 8, 8, 4]
 
 
 def test_edges(shape):
