@@ -724,7 +724,7 @@ uint64_t batch_sum(const std::vector<GateJob> &jobs, uint64_t per) {
 // for a round, in a second one of a shape of their own: spread evenly over all SMs in the smallest variant
 // that holds them, or in the latency form when that is one gate per SM. (In the last round of one launch
 // they held a few SMs for a full round while the others idled. B200, one launch -> this: 1300 BABYBEAR
-// gates 48.2 -> 29.3 ms, 2500 BABYBEAR 72.3 -> 53.8, 600 GOLDILOCKS 92.4 -> 56.4.)
+// gates 48.2 -> 28.5 ms, 2500 BABYBEAR 72.3 -> 52.4, 600 GOLDILOCKS 92.4 -> 55.7.)
 int run_rounds(hb_ctx *ctx, hb_keys *keys, std::vector<GateJob> jobs) {
   const uint32_t tuned = (uint32_t)keys->gates_per_cta;
   const bool tensor = tc_applies(ctx, keys->p, keys->threads_per_gate, (int)tuned);

@@ -13,9 +13,9 @@
 //
 // What bounds it: the integer pipes. Per transformed word a thread issues about 20 instructions for each
 // recombination, 19 for the twist between the passes and 31 for the products with both key polynomials;
-// the butterfly network of bootstrap_kernel issues about 160 and 34. ncu, 592 gates: ALU 55 %,
-// multiply pipe 53 %, tensor core 10 % of the time. Measured on B200, one wave of 592 gates: GOLDILOCKS 64.1 ->
-// 46.1 ms, ZAMA 99 -> 69.8 ms. For the 32-bit
+// the butterfly network of bootstrap_kernel issues about 160 and 34. ncu, 592 gates: ALU 56 %,
+// multiply pipe 54 %, tensor core 10 % of the time. Measured on B200, one wave of 592 gates: GOLDILOCKS 63.7 ->
+// 45.7 ms, ZAMA 97.5 -> 69.3 ms. For the 32-bit
 // fields, whose butterflies are 8 to 11 instructions, the same form measured no faster than bootstrap_kernel
 // (BABYBEAR 12.8 against 12.4 ms), so it is built for Goldilocks only.
 #pragma once

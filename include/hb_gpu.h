@@ -324,8 +324,8 @@ uint64_t hb_ctx_launches(const hb_ctx *ctx);
  * No counterpart in the reference. */
 int hb_ctx_set_wait_limit(hb_ctx *ctx, long long clock_cycles);
 /* Test hook for the path above: while on, bootstrapping launches and the tensor-core external
- * products of this context issue no key copies, so their first wait for a key chunk runs out (a flag that nothing sets) and the call
- * returns HB_ERR_TIMEOUT. No counterpart in the reference. */
+ * products of this context issue no key copies, so their first wait for a key chunk runs out (a flag
+ * that nothing sets) and the call returns HB_ERR_TIMEOUT. No counterpart in the reference. */
 int hb_ctx_test_withhold_keys(hb_ctx *ctx, int on);
 
 #ifdef __cplusplus
